@@ -105,7 +105,7 @@ struct cgs_ctx {
     bool drec_valid = false;
     bool kahan = false;          // compensated spreading (cgs_set_precision)
     // launch shapes (cgs_autotune): coils per spreading block (0: as many as
-    // fit), coils per interpolation thread
+    // fit), coils per interpolation thread (0: 2)
     int spread_cc = 0;
     int spread_wpp = 8;          // spreading variant: warps per x plane 1 / 2, 3 atomics, 4 / 5 pipelined,
                                  // 6 / 7 gather over the transposed tap matrix, staged in shared memory /
@@ -113,7 +113,7 @@ struct cgs_ctx {
                                  // fused with the adjoint x pass (6 where that does not apply)
     bool deterministic = true;   // fixed summation order everywhere (cgs_set_deterministic)
     bool spread_fused = false;   // the last adjoint half ran the fused spreading + x pass
-    int interp_cc = 4;
+    int interp_cc = 0;
     bool k_host_stale = false;   // d_k updated on the device (cgs_update_trajectory_d)
     uint64_t traj_serial = 0;    // incremented whenever the coordinates change
     bool tiles_stale = false;    // spreading lists built from older coordinates
@@ -129,6 +129,10 @@ struct cgs_ctx {
     DevBuf d_sup_rowmask;
     long long sup_rowmask_bs = 0;            // words per bin (0: not built)
     int sup_tb = 0;                          // columns per listed x-pass tile (fft_listed_cols)
+    // touch mask of the forward x pass over quads of coils (FwdXQuadArgs), in
+    // words per listed tile; 0: not built (every point of a listed tile is stored)
+    DevBuf d_touch;
+    int touch_words = 0;
     // the spreading gather's listing (variants 6, 7): tiles of the strided
     // passes' width, each a union of x-pass tiles, so that it stores every
     // column the adjoint x pass reads, in 128-byte rows
@@ -519,6 +523,40 @@ bool fused_spread_applies(const cgs_ctx* c)
     return !(cc == 2 || cc == 4 || cc == 6) || c->nch % cc == 0;
 }
 
+// The forward grid holds quads of coils (fwd_x_quad.cuh) from three coils on;
+// with one or two, coil planes (a quad would be mostly padding).
+bool quad_grid(const cgs_ctx* c) { return c->nch >= 3; }
+// values of a bin's forward grid
+long long fwd_grid_elems(const cgs_ctx* c)
+{
+    return (quad_grid(c) ? 4LL * ((c->nch + 3) / 4) : (long long)c->nch) * c->Ng;
+}
+
+// Touch mask of the listed x-pass tiles, from the transposed tap matrix over
+// either listing (a point's taps do not depend on the listing)
+int build_touch_mask(cgs_ctx* c)
+{
+    c->touch_words = 0;
+    if (!quad_grid(c) || !c->sup_built || !c->csr_valid || c->h_sup_off[c->nbins] == 0) return CGS_OK;
+    TouchMaskArgs a{};
+    a.tbq = fft_quad_cols(c->G[0], c->lo[0], c->I[0], &a.R1, &a.R2);
+    if (a.tbq <= 0 || c->sup_tb % a.tbq != 0) return CGS_OK;
+    a.nsub = c->sup_tb / a.tbq;
+    a.tiles = c->d_sup_tiles.as<int2>();
+    a.ntl = c->h_sup_off[c->nbins];
+    const int words = a.nsub * a.R1 * ((a.R2 + 3) / 4);
+    CGS_CUDA(c, c->d_touch.ensure((size_t)a.ntl * words * sizeof(unsigned)));
+    a.col_tile = c->d_col_tile.as<int>();
+    a.tb = c->csr_list == 1 ? c->sup_tb : c->spr_tb;
+    a.Gx = c->G[0];
+    a.ncol = (long long)c->G[1] * c->G[2];
+    a.ptr = c->d_csr_ptr.as<unsigned>();
+    a.mask = c->d_touch.as<unsigned>();
+    CGS_CUDA(c, launch_touch_mask(a, c->stream));
+    c->touch_words = words;
+    return CGS_OK;
+}
+
 // The transposed tap matrix over the listing the current spreading variant
 // reads (rebuilt, and the captured graphs dropped, when it changes)
 int ensure_csr(cgs_ctx* c)
@@ -654,7 +692,9 @@ int rebuild_bins(cgs_ctx* c)
     c->setup_ms[2] = ms_since(t0);
     t0 = clk::now();
     c->csr_list = -1;
+    c->touch_words = 0;
     CGS_TRY(ensure_csr(c));
+    CGS_TRY(build_touch_mask(c));
     c->setup_ms[3] = ms_since(t0);
     t0 = clk::now();
     std::vector<int> tile_ptr;
@@ -680,7 +720,8 @@ int rebuild_bins(cgs_ctx* c)
     }
     CGS_CUDA(c, c->d_yv.ensure(std::max<long long>(c->total, 1) * c->nch * sizeof(float2)));
     // workspace for a group of bins
-    const long long per_bin = (long long)c->nch * (c->Nl * c->G[2] + 2LL * c->I[0] * c->G[1] * c->G[2] + c->Ng) *
+    const long long grid_elems = fwd_grid_elems(c);
+    const long long per_bin = ((long long)c->nch * (c->Nl * c->G[2] + 2LL * c->I[0] * c->G[1] * c->G[2]) + grid_elems) *
                               (long long)sizeof(float2);
     long long budget = c->p.workspace_bytes > 0 ? c->p.workspace_bytes : (64LL << 30);
     int wsb = (int)std::max<long long>(1, std::min<long long>(c->nbins, budget / std::max<long long>(per_bin, 1)));
@@ -690,7 +731,7 @@ int rebuild_bins(cgs_ctx* c)
     CGS_CUDA(c, c->d_ybuf.ensure(wsn * (long long)c->I[0] * c->G[1] * c->G[2] * sizeof(float2)));
     CGS_CUDA(c, c->d_ybuf_adj.ensure(wsn * (long long)c->I[0] * c->G[1] * c->G[2] * sizeof(float2)));
     c->adj_slot.assign(c->ws_bins, -1);
-    CGS_CUDA(c, c->d_grid.ensure(wsn * c->Ng * sizeof(float2)));
+    CGS_CUDA(c, c->d_grid.ensure(c->ws_bins * grid_elems * sizeof(float2)));
     CGS_CUDA(c, cudaStreamSynchronize(c->stream));
     c->setup_ms[4] = ms_since(t0);   // the remaining lists' uploads and the workspaces
     c->toep_valid = false;
@@ -747,10 +788,11 @@ void set_cg_fusion(const cgs_ctx* c, FwdZArgs& fz, int b0, const float2* x)
     fz.cg_x = c->cgf.x + off;
 }
 
-// Forward half for bins [b0, b0+nb) (nb <= ws_bins): image(s) -> grid -> samples (yv).
+// Forward half for bins [b0, b0+nb) (nb <= ws_bins): image(s) -> grid -> samples
+// (yv; not with interp false: the caller reads the grid itself).
 // x: per bin [Ni] (x_bs) shared by the coils, or per coil (x_cs) without coil maps.
 int fwd_chain(cgs_ctx* c, int b0, int nb, const float2* x, long long x_bs, long long x_cs, bool use_smaps,
-              bool use_dcf)
+              bool use_dcf, bool interp = true)
 {
     const int Ix = c->I[0], Iy = c->I[1], Iz = c->I[2];
     const int Gx = c->G[0], Gy = c->G[1], Gz = c->G[2];
@@ -801,27 +843,49 @@ int fwd_chain(cgs_ctx* c, int b0, int nb, const float2* x, long long x_bs, long 
     }
     CGS_LAUNCH(c, launch_strided(Gy, -1, fy, Ix, nb * c->nch, c->stream));
 
-    StridedPassArgs fx{};
-    fx.in = c->d_ybuf.as<float2>();
-    fx.out = c->d_grid.as<float2>();
-    fx.in_bs = yb;
-    fx.out_bs = c->Ng;
-    fx.in_as = 0;
-    fx.out_as = 0;
-    fx.B = Gy * Gz;
-    fx.Lin = Ix;
-    fx.in_off = c->lo[0];
-    fx.Lout = Gx;
-    fx.out_off = 0;
-    fx.err = c->d_err.as<int>();
-    fx.tw = c->tw[0].as<float2>();
-    if (sup) set_support_tiles(c, fx, b0, nb);
-    CGS_LAUNCH(c, launch_strided(Gx, -1, fx, 1, nb * c->nch, c->stream));
+    if (quad_grid(c)) {
+        FwdXQuadArgs fx{};
+        fx.in = c->d_ybuf.as<float2>();
+        fx.in_bs = yb;
+        fx.out = c->d_grid.as<float2>();
+        fx.Ng = c->Ng;
+        fx.B = Gy * Gz;
+        fx.Lin = Ix;
+        fx.in_off = c->lo[0];
+        fx.nch = c->nch;
+        fx.nbins = nb;
+        fx.bin0 = b0;
+        if (sup) {
+            fx.tiles = c->d_sup_tiles.as<int2>() + c->h_sup_off[b0];
+            fx.ntl = c->h_sup_off[b0 + nb] - c->h_sup_off[b0];
+            fx.tb = c->sup_tb;
+            if (c->touch_words) fx.mask = c->d_touch.as<unsigned>() + c->h_sup_off[b0] * c->touch_words;
+        }
+        fx.tw = c->tw[0].as<float2>();
+        fx.err = c->d_err.as<int>();
+        CGS_LAUNCH(c, launch_fwd_x_quad(Gx, fx, c->stream));
+    } else {
+        StridedPassArgs fx{};
+        fx.in = c->d_ybuf.as<float2>();
+        fx.out = c->d_grid.as<float2>();
+        fx.in_bs = yb;
+        fx.out_bs = c->Ng;
+        fx.B = Gy * Gz;
+        fx.Lin = Ix;
+        fx.in_off = c->lo[0];
+        fx.Lout = Gx;
+        fx.err = c->d_err.as<int>();
+        fx.tw = c->tw[0].as<float2>();
+        if (sup) set_support_tiles(c, fx, b0, nb);
+        CGS_LAUNCH(c, launch_strided(Gx, -1, fx, 1, nb * c->nch, c->stream));
+    }
+    if (!interp) return CGS_OK;
 
     InterpArgs ia{};
     ia.grid = c->d_grid.as<float2>();
-    ia.coil_stride = c->Ng;
-    ia.grid_bs = (long long)c->nch * c->Ng;
+    ia.quad = quad_grid(c);
+    ia.coil_stride = ia.quad ? 4 * c->Ng : c->Ng;
+    ia.grid_bs = fwd_grid_elems(c);
     ia.rec = c->d_rec.as<TapRecord>();
     ia.dcf = (use_dcf && c->has_dcf) ? c->d_dcf_sorted.as<float>() : nullptr;
     ia.bin_off = c->d_bin_off.as<long long>();
@@ -1445,8 +1509,9 @@ int ensure_grad_records(cgs_ctx* c)
 PairGradArgs pair_args(const cgs_ctx* c, int b, int slot)
 {
     PairGradArgs pa{};
-    pa.grid = c->d_grid.as<float2>() + (long long)slot * c->nch * c->Ng;
-    pa.coil_stride = c->Ng;
+    pa.grid = c->d_grid.as<float2>() + (long long)slot * fwd_grid_elems(c);
+    pa.quad = quad_grid(c);
+    pa.coil_stride = pa.quad ? 4 * c->Ng : c->Ng;
     pa.rec = c->d_rec.as<TapRecord>();
     pa.drec = c->d_drec.as<TapRecord>();
     pa.dcf = c->has_dcf ? c->d_dcf_sorted.as<float>() : nullptr;
@@ -2291,18 +2356,19 @@ int cgs_loss_grad_d(cgs_ctx* c, int32_t bin, const void* x, const void* y, doubl
     if (bin < 0 || bin >= c->nbins) return fail(c, CGS_ERR_ARG, "bin out of range");
     const long long s0 = c->h_bin_off[bin], n = c->h_bin_off[bin + 1] - s0;
     CGS_TRY(ensure_grad_records(c));
-    // forward chain of the bin: every coil's grid (the interpolation it ends
-    // with is recomputed below together with the derivatives)
-    CGS_TRY(fwd_chain(c, bin, 1, reinterpret_cast<const float2*>(x), 0, 0, true, false));
+    // forward chain of the bin up to every coil's grid (the samples are
+    // interpolated below, together with the derivatives)
+    CGS_TRY(fwd_chain(c, bin, 1, reinterpret_cast<const float2*>(x), 0, 0, true, false, false));
     CGS_CUDA(c, c->d_gy.ensure(std::max<long long>(c->total, 1) * c->nch * sizeof(float2)));
     CGS_CUDA(c, launch_gather_samples(reinterpret_cast<const float2*>(y), c->ns, c->d_sorted.as<int>() + s0, n, c->nch,
                                       nullptr, c->d_gy.as<float2>() + s0 * c->nch, c->stream));
-    const int nblk = interp_grad_blocks(n);
+    const int nblk = interp_grad_blocks(n, quad_grid(c));
     CGS_CUDA(c, c->d_gpart.ensure((size_t)nblk * sizeof(double)));
     if (grad_k) CGS_CUDA(c, cudaMemsetAsync(grad_k, 0, (size_t)(3 * c->ns) * sizeof(float), c->stream));
     InterpGradArgs ga{};
     ga.grid = c->d_grid.as<float2>();
-    ga.coil_stride = c->Ng;
+    ga.quad = quad_grid(c);
+    ga.coil_stride = ga.quad ? 4 * c->Ng : c->Ng;
     ga.rec = c->d_rec.as<TapRecord>();
     ga.drec = c->d_drec.as<TapRecord>();
     ga.ymeas = c->d_gy.as<float2>();
@@ -2524,7 +2590,7 @@ int cgs_apply_vjp_k_d(cgs_ctx* c, int32_t bin0, int32_t nb, const void* p, const
         const int n = std::min(c->ws_bins, bin0 + nb - g);
         const long long off = (long long)(g - bin0) * c->Ni;
         // pass 1: A = E S p and its derivatives, stored per sample
-        CGS_TRY(fwd_chain(c, g, n, P + off, c->Ni, 0, true, false));
+        CGS_TRY(fwd_chain(c, g, n, P + off, c->Ni, 0, true, false, false));
         for (int b = g; b < g + n; ++b) {
             PairGradArgs pa = pair_args(c, b, b - g);
             pa.outA = c->d_pa.as<float2>();
@@ -2532,7 +2598,7 @@ int cgs_apply_vjp_k_d(cgs_ctx* c, int32_t bin0, int32_t nb, const void* p, const
             CGS_LAUNCH(c, launch_pair_grad(pa, c->stream));
         }
         // pass 2: B = E S v, contracted with (A, dA)
-        CGS_TRY(fwd_chain(c, g, n, V + off, c->Ni, 0, true, false));
+        CGS_TRY(fwd_chain(c, g, n, V + off, c->Ni, 0, true, false, false));
         for (int b = g; b < g + n; ++b) {
             PairGradArgs pa = pair_args(c, b, b - g);
             pa.A = c->d_pa.as<float2>();
@@ -2557,7 +2623,7 @@ int cgs_rhs_vjp_k_d(cgs_ctx* c, int32_t bin0, int32_t nb, const void* y, const v
     const float2* V = reinterpret_cast<const float2*>(v);
     for (int g = bin0; g < bin0 + nb; g += c->ws_bins) {
         const int n = std::min(c->ws_bins, bin0 + nb - g);
-        CGS_TRY(fwd_chain(c, g, n, V + (long long)(g - bin0) * c->Ni, c->Ni, 0, true, false));
+        CGS_TRY(fwd_chain(c, g, n, V + (long long)(g - bin0) * c->Ni, c->Ni, 0, true, false, false));
         for (int b = g; b < g + n; ++b) {
             PairGradArgs pa = pair_args(c, b, b - g);
             pa.A = c->d_gy.as<float2>();
@@ -2727,7 +2793,7 @@ int cgs_pipe_menon_dcf(cgs_ctx* c, int32_t iters, float* dcf, int32_t on_device)
             ia.thresh = c->thresh;
             long long mx = 0;
             for (int b = g; b < g + nb; ++b) mx = std::max(mx, c->h_bin_off[b + 1] - c->h_bin_off[b]);
-            CGS_LAUNCH(c, launch_interp(ia, mx, nb, 2, c->stream));
+            CGS_LAUNCH(c, launch_interp(ia, mx, nb, 0, c->stream));
         }
         CGS_CUDA(c, launch_pm_update(w.as<float>(), v.as<float2>(), u.as<float2>(), n, c->stream));
     }

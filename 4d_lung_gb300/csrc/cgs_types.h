@@ -64,6 +64,27 @@ struct StridedPassArgs {
     int sup_rowmask_tb;
 };
 
+// Forward x pass into the quad grid (fwd_x_quad.cuh): input item
+// slot * nch + c of Lin rows of B columns, output sector of point p of quad q
+// at out + ((slot * ceil(nch / 4) + q) * Ng + p) * 4.
+struct FwdXQuadArgs {
+    const float2* in;
+    long long in_bs;           // item stride
+    float2* out;
+    long long Ng;
+    int B, Lin, in_off;
+    int nch, nbins;            // bins of this launch (workspace slots 0 .. nbins - 1)
+    const int2* tiles;         // listed tiles {bin, first column} of this launch, or null: all columns
+    long long ntl;             // listed tiles
+    int tb;                    // columns per listed tile
+    int bin0;                  // bin of workspace slot 0
+    // touch mask of the listed tiles, or null: per tile and sub-tile of
+    // fft_quad_cols columns, per k1 ceil(R2 / 4) words: byte k2, bit column
+    const unsigned* mask;
+    const float2* tw;
+    int* err;
+};
+
 struct ContigPassArgs {
     const float2* in;
     float2* out;
@@ -130,8 +151,9 @@ struct KbParams {
 };
 
 struct InterpArgs {
-    const float2* grid;        // coil c at grid + c*coil_stride (+ bin stride)
-    long long coil_stride;
+    const float2* grid;        // coil c at grid + c*coil_stride (+ bin stride), or quads of coils:
+    long long coil_stride;     //   quad q at grid + q*coil_stride, point p and coil c of it at 4 p + c
+    bool quad;
     long long grid_bs;         // bin stride of the grids (blockIdx.z)
     const TapRecord* rec;      // sorted tap records (all bins concatenated)
     const float* dcf;          // sorted density weights, or null
@@ -189,6 +211,21 @@ struct CsrBuildArgs {
     const unsigned* ptr;       // [P + 1] row offsets (fill pass)
     int2* ent;                 // {sorted sample, weight bits} (fill pass)
     int* err;                  // set when a tap lands outside the listed columns
+};
+
+// Touch mask of the listed x-pass tiles (FwdXQuadArgs::mask) from the row
+// offsets of the transposed tap matrix: a point's bit is set when it has taps.
+struct TouchMaskArgs {
+    const int2* tiles;         // listed x-pass tiles {bin, first column}, all bins
+    long long ntl;
+    int nsub, tbq;             // sub-tiles per listed tile, columns of each
+    int R1, R2;                // split of the x line
+    const int* col_tile;       // of the matrix's listing (CsrBuildArgs)
+    int tb;                    // columns per tile of that listing
+    int Gx;
+    long long ncol;            // Gy * Gz
+    const unsigned* ptr;
+    unsigned* mask;
 };
 
 struct CsrSpreadArgs {
@@ -258,8 +295,9 @@ struct PsfSpreadArgs {
 
 // Loss gradient pass (grad.cu): one bin's samples [s0, s0 + n) in sorted order.
 struct InterpGradArgs {
-    const float2* grid;        // coil c at grid + c * coil_stride (one bin)
+    const float2* grid;        // one bin's grid, as in InterpArgs
     long long coil_stride;
+    bool quad;
     const TapRecord* rec;      // tap records (sorted order)
     const TapRecord* drec;     // derivative records (sorted order)
     const float2* ymeas;       // measured samples [sorted][nch]
@@ -281,8 +319,9 @@ struct InterpGradArgs {
 //   contract mode: grad_k[g] += scale D_i Re sum_c (conj(B) dA + conj(dB) A)
 //                  (dA may be null: a fixed first factor such as measured data)
 struct PairGradArgs {
-    const float2* grid;
+    const float2* grid;        // as in InterpArgs
     long long coil_stride;
+    bool quad;
     const TapRecord* rec;
     const TapRecord* drec;
     const float2* A;           // [sorted][nch]

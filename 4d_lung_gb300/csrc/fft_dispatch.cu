@@ -14,7 +14,8 @@ namespace cgs {
     cudaError_t fft_init_##L_();                                                                       \
     cudaError_t fft_toep_x_##L_(const StridedPassArgs& a, const float* P, long long p_bs, int nsub, int batch, \
                                 cudaStream_t s);                                                       \
-    cudaError_t fft_spread_adjx_##L_(const SpreadAdjxArgs& a, bool kahan, cudaStream_t s);
+    cudaError_t fft_spread_adjx_##L_(const SpreadAdjxArgs& a, bool kahan, cudaStream_t s);             \
+    cudaError_t fft_fwd_x_quad_##L_(const FwdXQuadArgs& a, cudaStream_t s);
 CGS_FFT_SIZES(CGS_DECLARE)
 
 static const int kSizes[] = {
@@ -83,6 +84,23 @@ bool encode_strided_map(CUtensorMap* map, const StridedPassArgs& a, int A, int b
     return true;
 }
 
+bool encode_items_map(CUtensorMap* map, const float2* in, int B, int Lin, long long item_stride, long long items,
+                      int TB, int box_rows, int promo)
+{
+    if ((reinterpret_cast<uintptr_t>(in) & 15) || (B & 1) || (item_stride & 1) || Lin < 1 || box_rows > 256) return false;
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)B, (cuuint64_t)Lin, 1, (cuuint64_t)items};
+    const cuuint64_t strides[3] = {(cuuint64_t)B * 8, (cuuint64_t)item_stride * 8, (cuuint64_t)item_stride * 8};
+    const cuuint32_t box[4] = {(cuuint32_t)TB, (cuuint32_t)box_rows, 1, 1};
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    const CUtensorMapL2promotion pr =
+        promo <= 64 ? CU_TENSOR_MAP_L2_PROMOTION_L2_64B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B;
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<float2*>(in), dims, strides, box, es,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, pr,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool encode_spectrum_map(CUtensorMap* map, const float* P, long long B, int L, int nbins, int TB, int* box_rows)
 {
     // rows of 4-byte elements: base and row pitch on 16-byte boundaries
@@ -128,6 +146,21 @@ int fft_listed_cols(int L, int lo, int I)
     switch (L) {
 #define CGS_CASE(L_, R1_, R2_, G_) \
     case L_: return half ? fft_listed_tile_cols(R1_, R2_) : fft_strided_tile_cols(R1_, R2_);
+        CGS_FFT_SIZES(CGS_CASE)
+#undef CGS_CASE
+    }
+    return 0;
+}
+
+int fft_quad_cols(int L, int lo, int I, int* R1, int* R2)
+{
+    const bool half = 4 * lo == L && 2 * I == L;
+    switch (L) {
+#define CGS_CASE(L_, R1_, R2_, G_)                                                 \
+    case L_:                                                                       \
+        *R1 = R1_;                                                                 \
+        *R2 = R2_;                                                                 \
+        return fft_quad_tile_cols(R1_, R2_, half && R1_ % 4 == 0);
         CGS_FFT_SIZES(CGS_CASE)
 #undef CGS_CASE
     }
@@ -210,6 +243,16 @@ cudaError_t launch_spread_adjx(int L, const SpreadAdjxArgs& a, bool kahan, cudaS
 #undef CGS_CASE
     }
     return cudaErrorNotSupported;
+}
+
+cudaError_t launch_fwd_x_quad(int L, const FwdXQuadArgs& a, cudaStream_t s)
+{
+    switch (L) {
+#define CGS_CASE(L_, R1_, R2_, G_) case L_: return fft_fwd_x_quad_##L_(a, s);
+        CGS_FFT_SIZES(CGS_CASE)
+#undef CGS_CASE
+    }
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace cgs

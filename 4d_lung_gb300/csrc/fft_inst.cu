@@ -4,6 +4,7 @@
 #include "launch.h"
 #include "fft_passes.cuh"
 #include "spread_adjx.cuh"
+#include "fwd_x_quad.cuh"
 
 #ifndef CGS_FFT_GROUP
 #define CGS_FFT_GROUP 0
@@ -59,6 +60,8 @@ struct SizeImpl {
     // pipeline stages of the narrow forward pass: its stages hold half as
     // many bytes (Ix rows of 64 bytes), so one more keeps as many in flight
     static constexpr int NSTAGE_NI = 3;
+    // forward x pass over quads of coils: unit widths of the two forms
+    static constexpr int TBQ_IN = fft_quad_tile_cols(R1, R2, true), TBQ_NO = fft_quad_tile_cols(R1, R2, false);
 
     template <int SIGN, int MODE, int TBK = TB, int NS = NSTAGE>
     static cudaError_t tma_attr(int smem)
@@ -82,6 +85,15 @@ struct SizeImpl {
             if (e == cudaSuccess)
                 e = tma_attr<+1, PRUNE_OUT, TBN>((int)PipeLayout<R1, R2, TBN, NSTAGE>::smem_bytes(L));
         }
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_fwd_x_quad<R1, R2, TBQ_NO, PRUNE_NONE>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)QuadLayout<R1, R2, TBQ_NO>::smem_bytes(L + 3));
+        if constexpr (HAS_IN)
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k_fwd_x_quad<R1, R2, TBQ_IN, PRUNE_IN>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)QuadLayout<R1, R2, TBQ_IN>::smem_bytes(L / 2));
         if constexpr (HAS_IN)
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(k_toep_x_tma<R1, R2, TBT, NSTAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -166,6 +178,39 @@ struct SizeImpl {
         if (sign < 0) k_fft_strided<R1, R2, -1, TB><<<grid, NT_S, 0, s>>>(a);
         else k_fft_strided<R1, R2, +1, TB><<<grid, NT_S, 0, s>>>(a);
         return cudaGetLastError();
+    }
+    // forward x pass into the quad grid
+    template <int TBQ, int MODE>
+    static cudaError_t quad_run(const FwdXQuadArgs& a, cudaStream_t s)
+    {
+        using Q = QuadLayout<R1, R2, TBQ>;
+        // rows of the line in boxes of at most 256, all of one size
+        const int nbox = (a.Lin + 255) / 256;
+        const int box_rows = nbox == 1 ? a.Lin : (((a.Lin + nbox - 1) / nbox) + 3) & ~3;
+        CUtensorMap map;
+        if (!encode_items_map(&map, a.in, a.B, a.Lin, a.in_bs, (long long)a.nbins * a.nch, TBQ, box_rows, TBQ * 8))
+            return cudaErrorNotSupported;
+        const size_t smem = Q::smem_bytes(nbox * box_rows);
+        int per_sm = 0;
+        cudaError_t e =
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fwd_x_quad<R1, R2, TBQ, MODE>, Q::NT, smem);
+        if (e != cudaSuccess) return e;
+        const int nsub = a.tiles ? a.tb / TBQ : (a.B + TBQ - 1) / TBQ;
+        const long long per_quad = (a.tiles ? a.ntl : (long long)a.nbins) * nsub;
+        const long long nunits = per_quad * ((a.nch + 3) / 4);
+        if (nunits <= 0) return cudaSuccess;   // no listed tile: nothing to transform
+        if (nunits >= 0x7fffffffLL) return cudaErrorInvalidValue;
+        const long long nblk = std::min<long long>(nunits, (long long)sm_count() * std::max(per_sm, 1));
+        k_fwd_x_quad<R1, R2, TBQ, MODE><<<(unsigned)nblk, Q::NT, smem, s>>>(a, map, (int)nunits, (int)per_quad, nsub,
+                                                                           box_rows, nbox);
+        return cudaGetLastError();
+    }
+    static cudaError_t fwd_x_quad(const FwdXQuadArgs& a, cudaStream_t s)
+    {
+        if (!a.err || a.nch < 1 || (a.tiles && a.tb % TBQ_IN != 0)) return cudaErrorInvalidValue;
+        if constexpr (HAS_IN)
+            if (4 * a.in_off == L && 2 * a.Lin == L) return quad_run<TBQ_IN, PRUNE_IN>(a, s);
+        return quad_run<TBQ_NO, PRUNE_NONE>(a, s);
     }
     // Toeplitz x stage (in place, rows L/4 .. 3L/4 in and out)
     static cudaError_t toep_x(StridedPassArgs a, const float* P, long long p_bs, int nsub, int batch, cudaStream_t s)
@@ -291,6 +336,7 @@ struct SizeImpl {
     cudaError_t fft_toep_x_##L_(const StridedPassArgs& a, const float* P, long long p_bs, int nsub, int batch, \
                                 cudaStream_t s);                                                       \
     cudaError_t fft_spread_adjx_##L_(const SpreadAdjxArgs& a, bool kahan, cudaStream_t s);             \
+    cudaError_t fft_fwd_x_quad_##L_(const FwdXQuadArgs& a, cudaStream_t s);                            \
     CGS_DEFINE_IF_##G_(L_, R1_, R2_)
 
 #define CGS_BODY(L_, R1_, R2_)                                                                      \
@@ -308,7 +354,9 @@ struct SizeImpl {
                                 cudaStream_t s)                                                        \
     { return SizeImpl<R1_, R2_>::toep_x(a, P, p_bs, nsub, batch, s); }                                \
     cudaError_t fft_spread_adjx_##L_(const SpreadAdjxArgs& a, bool kahan, cudaStream_t s)              \
-    { return SizeImpl<R1_, R2_>::spread_adjx(a, kahan, s); }
+    { return SizeImpl<R1_, R2_>::spread_adjx(a, kahan, s); }                                         \
+    cudaError_t fft_fwd_x_quad_##L_(const FwdXQuadArgs& a, cudaStream_t s)                             \
+    { return SizeImpl<R1_, R2_>::fwd_x_quad(a, s); }
 
 #if CGS_FFT_GROUP == 0
 #define CGS_DEFINE_IF_0(L, R1, R2) CGS_BODY(L, R1, R2)

@@ -22,6 +22,12 @@ constexpr int fft_listed_tile_cols(int r1, int r2)
     return fft_has_narrow_tiles(r1, r2) ? 8 : fft_strided_tile_cols(r1, r2);
 }
 
+// columns of a unit of the forward x pass over quads of coils (fwd_x_quad.cuh)
+constexpr int fft_quad_tile_cols(int r1, int r2, bool half_in)
+{
+    return (r1 > r2 ? r1 : r2) > 16 || (!half_in && r1 * r2 >= 160) ? 4 : 8;
+}
+
 // spreading fused with the adjoint x pass (spread_adjx.cuh): threads per
 // block, columns per tile (the x passes' narrow tiles)
 constexpr int SAX_NT = 1024, SAX_TB = 8;

@@ -157,11 +157,179 @@ __global__ void __launch_bounds__(128) k_interp_grad(InterpGradArgs a)
     if (threadIdx.x == 0) a.partials[blockIdx.x] = s_red[0] + s_red[1] + s_red[2] + s_red[3];
 }
 
-int interp_grad_blocks(long long n) { return (int)std::max<long long>((n + 127) / 128, 1); }
+// ---------------------------------------------------------------------------
+// The same passes over the quad grid (fwd_x_quad.cuh): four lanes per sample,
+// one coil of the quad each, so that a warp's load of one tap takes one
+// 32-byte sector per sample.  A lane adds its coil's value and derivatives
+// over the taps in the order of the kernels above with the same products and
+// tests, and the coil sums run in coil order: the same bits.  1 572 864
+// samples, 12 coils: k_interp_grad 7.93 -> 3.31 ms (its multiply-adds and the
+// weights formed anew per quad bound it now); 262 144 samples in four bins, 8
+// coils: k_pair_grad 0.36 -> 0.11 ms a launch.
+// ---------------------------------------------------------------------------
+struct GradSums {
+    float2 y, d0, d1, d2;
+};
+
+// A sample's factors and their derivatives.  Where all three supports of every
+// sample of the warp hold exactly four candidates, these are moved to the
+// positions 0 .. 3 of each axis (`four`), else candidates sit at 0 .. 4.
+struct QuadTaps {
+    float w[15], dw[15];
+    long long base;   // grid point of candidate (0, 0, 0); may lie outside the grid unless four
+    bool four;
+};
+
+// all 32 lanes of the warp
+CGS_D void quad_taps(const TapRecord* rec, const TapRecord* drec, long long i, int Gy, int Gz, QuadTaps& t)
+{
+    int nx, ny, nz, t0, t1, t2;
+    load_record(rec, i, t.w, nx, ny, nz);
+    load_record(drec, i, t.dw, t0, t1, t2);
+    bool ok = true;
+    int sh[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float* w = t.w + 5 * a;
+        sh[a] = w[0] == 0.f;
+        ok = ok && w[1] != 0.f && w[2] != 0.f && w[3] != 0.f && ((w[0] == 0.f) != (w[4] == 0.f));
+    }
+    t.four = __all_sync(0xffffffffu, ok);
+    if (t.four) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                t.w[5 * a + q] = sh[a] ? t.w[5 * a + q + 1] : t.w[5 * a + q];
+                t.dw[5 * a + q] = sh[a] ? t.dw[5 * a + q + 1] : t.dw[5 * a + q];
+            }
+        nx += sh[0];
+        ny += sh[1];
+        nz += sh[2];
+    }
+    t.base = ((long long)(nx - 2) * Gy + (ny - 2)) * Gz + (nz - 2);
+}
+
+// The compiler must not keep the 125 taps' weights across the coils (it would
+// spill them): each coil's sums form them anew from the 30 factors.
+CGS_D void opaque(QuadTaps& t)
+{
+#pragma unroll
+    for (int q = 0; q < 15; ++q) asm volatile("" : "+f"(t.w[q]), "+f"(t.dw[q]));
+}
+
+// Value and coordinate derivatives of one coil at one sample; g: the coil's
+// first point (points 4 apart)
+template <int N>
+CGS_D GradSums quad_grad_run(const float2* __restrict__ g, const QuadTaps& t, int Gy, int Gz, float thresh)
+{
+    GradSums r;
+    r.y = r.d0 = r.d1 = r.d2 = make_float2(0.f, 0.f);
+    const float2* b = g + t.base * 4;
+#pragma unroll
+    for (int jx = 0; jx < N; ++jx)
+#pragma unroll
+        for (int y0 = 0; y0 < N; y0 += N == 4 ? 4 : 1) {
+            constexpr int NY = N == 4 ? 4 : 1;
+            float2 v[NY][N];
+#pragma unroll
+            for (int q = 0; q < NY; ++q) {
+                const float2* row = b + (long long)(jx * Gy + y0 + q) * Gz * 4;
+                const float wxy = t.w[jx] * t.w[5 + y0 + q];
+#pragma unroll
+                for (int jz = 0; jz < N; ++jz)   // with N = 4 every candidate lies in the grid
+                    if (N == 4 || wxy * t.w[10 + jz] > thresh) v[q][jz] = __ldg(row + jz * 4);
+            }
+#pragma unroll
+            for (int q = 0; q < NY; ++q) {
+                const float wx = t.w[jx], dwx = t.dw[jx], wy = t.w[5 + y0 + q], dwy = t.dw[5 + y0 + q];
+                const float wxy = wx * wy, ax = dwx * wy, ay = wx * dwy;
+#pragma unroll
+                for (int jz = 0; jz < N; ++jz) {
+                    const float wz = t.w[10 + jz], dwz = t.dw[10 + jz];
+                    const float wt = wxy * wz;   // 0 outside the support or the grid
+                    if (wt > thresh) {
+                        const float ex = ax * wz, ey = ay * wz, ez = wxy * dwz;
+                        r.y.x = fmaf(v[q][jz].x, wt, r.y.x);
+                        r.y.y = fmaf(v[q][jz].y, wt, r.y.y);
+                        r.d0.x = fmaf(v[q][jz].x, ex, r.d0.x);
+                        r.d0.y = fmaf(v[q][jz].y, ex, r.d0.y);
+                        r.d1.x = fmaf(v[q][jz].x, ey, r.d1.x);
+                        r.d1.y = fmaf(v[q][jz].y, ey, r.d1.y);
+                        r.d2.x = fmaf(v[q][jz].x, ez, r.d2.x);
+                        r.d2.y = fmaf(v[q][jz].y, ez, r.d2.y);
+                    }
+                }
+            }
+        }
+    return r;
+}
+CGS_D GradSums quad_grad_sums(const float2* __restrict__ g, const QuadTaps& t, int Gy, int Gz, float thresh)
+{
+    return t.four ? quad_grad_run<4>(g, t, Gy, Gz, thresh) : quad_grad_run<5>(g, t, Gy, Gz, thresh);
+}
+
+constexpr int QG_SAMPLES = 32;   // samples per block of 128 threads
+
+__global__ void __launch_bounds__(4 * QG_SAMPLES) k_interp_grad_quad(InterpGradArgs a)
+{
+    __shared__ double s_red[QG_SAMPLES / 8];
+    const int lane = threadIdx.x & 31, sub = threadIdx.x & 3, lead = lane & ~3;
+    const long long j = (long long)blockIdx.x * QG_SAMPLES + threadIdx.x / 4;
+    const bool on = j < a.n;
+    double loss = 0.0;
+    float gk0 = 0.f, gk1 = 0.f, gk2 = 0.f;
+    const long long i = a.s0 + (on ? j : 0);
+    if (a.n > 0) {
+        QuadTaps t;
+        quad_taps(a.rec, a.drec, i, a.G[1], a.G[2], t);
+        const float D = a.dcf ? a.dcf[i] : 1.f;
+        for (int c0 = 0; c0 < a.nch; c0 += 4) {
+            const int c = c0 + sub;
+            opaque(t);
+            const GradSums r = quad_grad_sums(a.grid + (long long)(c0 / 4) * a.coil_stride + sub, t, a.G[1], a.G[2],
+                                              a.thresh);
+            float p0 = 0.f, p1 = 0.f, p2 = 0.f;
+            if (on && c < a.nch) {
+                const float2 m = a.ymeas[i * a.nch + c];
+                const float rx = r.y.x - m.x, ry = r.y.y - m.y;
+                loss += 0.5 * (double)D * ((double)rx * rx + (double)ry * ry);
+                p0 = rx * r.d0.x + ry * r.d0.y;
+                p1 = rx * r.d1.x + ry * r.d1.y;
+                p2 = rx * r.d2.x + ry * r.d2.y;
+                if (a.rv) a.rv[i * a.nch + c] = make_float2(D * rx, D * ry);
+            }
+            // the quad's coils in order (every lane of the sample)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float b0 = __shfl_sync(0xffffffffu, p0, lead + q), b1 = __shfl_sync(0xffffffffu, p1, lead + q);
+                const float b2 = __shfl_sync(0xffffffffu, p2, lead + q);
+                if (c0 + q < a.nch) {
+                    gk0 = fmaf(D, b0, gk0);
+                    gk1 = fmaf(D, b1, gk1);
+                    gk2 = fmaf(D, b2, gk2);
+                }
+            }
+        }
+        if (a.grad_k && on && sub < 3) a.grad_k[3 * (long long)a.sorted[i] + sub] = sub == 0 ? gk0 : sub == 1 ? gk1 : gk2;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if (lane == 0) s_red[threadIdx.x >> 5] = loss;
+    __syncthreads();
+    if (threadIdx.x == 0) a.partials[blockIdx.x] = s_red[0] + s_red[1] + s_red[2] + s_red[3];
+}
+
+int interp_grad_blocks(long long n, bool quad)
+{
+    const int per = quad ? QG_SAMPLES : 128;
+    return (int)std::max<long long>((n + per - 1) / per, 1);
+}
 
 cudaError_t launch_interp_grad(const InterpGradArgs& a, cudaStream_t s)
 {
-    k_interp_grad<4><<<(unsigned)interp_grad_blocks(a.n), 128, 0, s>>>(a);
+    if (a.quad) k_interp_grad_quad<<<(unsigned)interp_grad_blocks(a.n, true), 4 * QG_SAMPLES, 0, s>>>(a);
+    else k_interp_grad<2><<<(unsigned)interp_grad_blocks(a.n, false), 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -267,9 +435,73 @@ __global__ void __launch_bounds__(128) k_pair_grad(PairGradArgs a)
     }
 }
 
+__global__ void __launch_bounds__(4 * QG_SAMPLES) k_pair_grad_quad(PairGradArgs a)
+{
+    const int lane = threadIdx.x & 31, sub = threadIdx.x & 3, lead = lane & ~3;
+    const long long j = (long long)blockIdx.x * QG_SAMPLES + threadIdx.x / 4;
+    const bool on = j < a.n;
+    const long long i = a.s0 + (on ? j : 0);
+    QuadTaps t;
+    quad_taps(a.rec, a.drec, i, a.G[1], a.G[2], t);
+    const float D = a.dcf ? a.dcf[i] : 1.f;
+    float gk[3] = {0.f, 0.f, 0.f};
+    for (int c0 = 0; c0 < a.nch; c0 += 4) {
+        const int c = c0 + sub;
+        opaque(t);
+        const GradSums r = quad_grad_sums(a.grid + (long long)(c0 / 4) * a.coil_stride + sub, t, a.G[1], a.G[2],
+                                          a.thresh);
+        const long long e = i * a.nch + c;
+        const bool mine = on && c < a.nch;
+        if (a.outA) {
+            if (mine) {
+                a.outA[e] = r.y;
+                a.outdA[3 * e + 0] = r.d0;
+                a.outdA[3 * e + 1] = r.d1;
+                a.outdA[3 * e + 2] = r.d2;
+            }
+            continue;
+        }
+        // Re(conj(B) dA + conj(dB) A), B = y, dB = d*, each product pair rounded
+        // as k_pair_grad rounds it
+        float p[3] = {0.f, 0.f, 0.f}, q[3] = {0.f, 0.f, 0.f};
+        if (mine) {
+            const float2 A = a.A[e];
+            p[0] = __fmaf_rn(A.x, r.d0.x, __fmul_rn(A.y, r.d0.y));
+            p[1] = __fmaf_rn(A.x, r.d1.x, __fmul_rn(A.y, r.d1.y));
+            p[2] = __fmaf_rn(A.x, r.d2.x, __fmul_rn(A.y, r.d2.y));
+            if (a.dA) {
+                const float2 e0 = a.dA[3 * e + 0], e1 = a.dA[3 * e + 1], e2 = a.dA[3 * e + 2];
+                q[0] = __fmaf_rn(r.y.x, e0.x, __fmul_rn(r.y.y, e0.y));
+                q[1] = __fmaf_rn(r.y.y, e1.y, __fmul_rn(r.y.x, e1.x));
+                q[2] = __fmaf_rn(r.y.x, e2.x, __fmul_rn(r.y.y, e2.y));
+            }
+        }
+        // the quad's coils in order (every lane of the sample)
+#pragma unroll
+        for (int l = 0; l < 4; ++l)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const float pl = __shfl_sync(0xffffffffu, p[d], lead + l), ql = __shfl_sync(0xffffffffu, q[d], lead + l);
+                if (c0 + l < a.nch) {
+                    gk[d] = __fadd_rn(gk[d], pl);
+                    if (a.dA) gk[d] = __fadd_rn(gk[d], ql);
+                }
+            }
+    }
+    if (a.outA || !on || sub >= 3) return;
+    const long long g = a.sorted[i];
+    const float f = a.scale * D;
+    const float sum = sub == 0 ? gk[0] : sub == 1 ? gk[1] : gk[2];
+    a.grad_k[3 * g + sub] += f * sum;
+}
+
 cudaError_t launch_pair_grad(const PairGradArgs& a, cudaStream_t s)
 {
     if (a.n == 0) return cudaSuccess;
+    if (a.quad) {
+        k_pair_grad_quad<<<(unsigned)((a.n + QG_SAMPLES - 1) / QG_SAMPLES), 4 * QG_SAMPLES, 0, s>>>(a);
+        return cudaGetLastError();
+    }
     k_pair_grad<2><<<(unsigned)((a.n + 127) / 128), 128, 0, s>>>(a);
     return cudaGetLastError();
 }

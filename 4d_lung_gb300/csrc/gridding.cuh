@@ -70,37 +70,46 @@ __global__ void k_tap_records(const double* __restrict__ k, const int* __restric
 // ---------------------------------------------------------------------------
 // Interpolation (Reco.cpp:539-550) fused with the density weights
 // (Reco.cpp:243-254):  yv[i][c] = D[i] * sum_taps w * grid_c[idx]
-// One thread per (sample, chunk of CC coils).  Grids are [coil][Ng]; the
-// sample values are written coil-interleaved, yv[i][c].
+// One thread per sample and coil, for grids of coil planes [coil][Ng] (one or
+// two coils); the sample values are written coil-interleaved, yv[i][c].
 // ---------------------------------------------------------------------------
 
-template <int CC>
 __global__ void __launch_bounds__(128) k_interp(InterpArgs a)
 {
     const int bin = a.bin0 + blockIdx.z;
     const long long s0 = a.bin_off[bin], s1 = a.bin_off[bin + 1];
-    // blockIdx.x = sample block * chunks + coil chunk: the chunks of a sample
-    // block run side by side, so the blocks in flight cover a short run of
-    // samples (a compact region of the grid) for all coils, which L2 holds
-    const int nchunk = (a.nch + CC - 1) / CC;
-    const int chunk = (int)(blockIdx.x % (unsigned)nchunk);
-    const long long i = s0 + (long long)(blockIdx.x / (unsigned)nchunk) * blockDim.x + threadIdx.x;
+    // blockIdx.x = sample block * coils + coil: the coils of a sample block
+    // run side by side, so the blocks in flight cover a short run of samples
+    // (a compact region of the grid) for all coils, which L2 holds
+    const int c = (int)(blockIdx.x % (unsigned)a.nch);
+    const long long i = s0 + (long long)(blockIdx.x / (unsigned)a.nch) * blockDim.x + threadIdx.x;
     if (i >= s1) return;
-    const int c0 = chunk * CC;
-    const float2* grid = a.grid + (long long)blockIdx.z * a.grid_bs + (long long)c0 * a.coil_stride;
+    const float2* grid = a.grid + (long long)blockIdx.z * a.grid_bs + (long long)c * a.coil_stride;
     float w[15];
     int nx, ny, nz;
     load_record(a.rec, i, w, nx, ny, nz);
-    float2 acc[CC];
-#pragma unroll
-    for (int c = 0; c < CC; ++c) acc[c] = make_float2(0.f, 0.f);
+    float2 acc = make_float2(0.f, 0.f);
     const int Gy = a.G[1], Gz = a.G[2];
-    const int ncc = min(CC, a.nch - c0);
     // Rows of 5 z taps away from the z edges are read as three aligned
     // 16-byte loads (6 points from the even index at or below the row's
     // first); grids and coil planes start on 16-byte boundaries (Ng even).
     const bool vec = nz >= 3 && nz + 3 <= Gz - 1 && (a.coil_stride & 1) == 0 &&
                      (reinterpret_cast<uintptr_t>(a.grid) & 15) == 0 && (a.grid_bs & 1) == 0;
+    auto add_row = [&](const float4* p, int odd, float wxy) {
+        const float4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2);
+        const float2 e[6] = {make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y),
+                             make_float2(q1.z, q1.w), make_float2(q2.x, q2.y), make_float2(q2.z, q2.w)};
+#pragma unroll
+        for (int jz = 0; jz < 5; ++jz) {
+            const float wz = w[10 + jz];
+            const float wt = wxy * wz;
+            if (wz != 0.f && wt > a.thresh) {
+                const float2 g = odd ? e[jz + 1] : e[jz];
+                acc.x = fmaf(g.x, wt, acc.x);
+                acc.y = fmaf(g.y, wt, acc.y);
+            }
+        }
+    };
     // Interior samples whose x and y supports hold exactly four candidates
     // each (a kernel of width 4 away from the grid points and the grid's
     // faces): a 4 x 4 loop over the rows without a branch per row, so that
@@ -132,85 +141,179 @@ __global__ void __launch_bounds__(128) k_interp(InterpArgs a)
 #pragma unroll
         for (int ix = 0; ix < 4; ++ix)
 #pragma unroll
-            for (int iy = 0; iy < 4; ++iy) {
-                const float wxy = wxs[ix] * wys[iy];
-                const float4* r4 = b4 + ix * gyz4 + iy * gz4;
-#pragma unroll
-                for (int c = 0; c < CC; ++c)
-                    if (c < ncc) {
-                        const float4* p = r4 + (long long)c * (a.coil_stride / 2);
-                        const float4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2);
-                        const float2 e[6] = {make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y),
-                                             make_float2(q1.z, q1.w), make_float2(q2.x, q2.y), make_float2(q2.z, q2.w)};
-#pragma unroll
-                        for (int jz = 0; jz < 5; ++jz) {
-                            const float wz = w[10 + jz];
-                            const float wt = wxy * wz;
-                            if (wz != 0.f && wt > a.thresh) {
-                                const float2 g = odd ? e[jz + 1] : e[jz];
-                                acc[c].x = fmaf(g.x, wt, acc[c].x);
-                                acc[c].y = fmaf(g.y, wt, acc[c].y);
-                            }
-                        }
-                    }
-            }
+            for (int iy = 0; iy < 4; ++iy) add_row(b4 + ix * gyz4 + iy * gz4, odd, wxs[ix] * wys[iy]);
     } else {
 #pragma unroll
-    for (int jx = 0; jx < 5; ++jx) {
-        const float wx = w[jx];
-        if (wx == 0.f) continue;
-        const int gx = nx - 2 + jx;
+        for (int jx = 0; jx < 5; ++jx) {
+            const float wx = w[jx];
+            if (wx == 0.f) continue;
+            const int gx = nx - 2 + jx;
 #pragma unroll
-        for (int jy = 0; jy < 5; ++jy) {
-            const float wxy = wx * w[5 + jy];
-            if (wxy == 0.f) continue;
-            const long long row = ((long long)gx * Gy + (ny - 2 + jy)) * Gz + (nz - 2);
-            if (vec) {
-                const int odd = (int)(row & 1);
-                const float4* r4 = reinterpret_cast<const float4*>(grid + (row - odd));
+            for (int jy = 0; jy < 5; ++jy) {
+                const float wxy = wx * w[5 + jy];
+                if (wxy == 0.f) continue;
+                const long long row = ((long long)gx * Gy + (ny - 2 + jy)) * Gz + (nz - 2);
+                if (vec) {
+                    const int odd = (int)(row & 1);
+                    add_row(reinterpret_cast<const float4*>(grid + (row - odd)), odd, wxy);
+                    continue;
+                }
 #pragma unroll
-                for (int c = 0; c < CC; ++c)
-                    if (c < ncc) {
-                        const float4* p = r4 + (long long)c * (a.coil_stride / 2);
-                        const float4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2);
-                        const float2 e[6] = {make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y),
-                                             make_float2(q1.z, q1.w), make_float2(q2.x, q2.y), make_float2(q2.z, q2.w)};
-#pragma unroll
-                        for (int jz = 0; jz < 5; ++jz) {
-                            const float wz = w[10 + jz];
-                            const float wt = wxy * wz;
-                            if (wz != 0.f && wt > a.thresh) {
-                                const float2 g = odd ? e[jz + 1] : e[jz];
-                                acc[c].x = fmaf(g.x, wt, acc[c].x);
-                                acc[c].y = fmaf(g.y, wt, acc[c].y);
-                            }
-                        }
+                for (int jz = 0; jz < 5; ++jz) {
+                    const float wz = w[10 + jz];
+                    const float wt = wxy * wz;
+                    if (wz != 0.f && wt > a.thresh) {   // wz != 0: the tap lies inside the grid
+                        const float2 g = __ldg(grid + row + jz);
+                        acc.x = fmaf(g.x, wt, acc.x);
+                        acc.y = fmaf(g.y, wt, acc.y);
                     }
-                continue;
-            }
-#pragma unroll
-            for (int jz = 0; jz < 5; ++jz) {
-                const float wz = w[10 + jz];
-                const float wt = wxy * wz;
-                if (wz != 0.f && wt > a.thresh) {   // wz != 0: the tap lies inside the grid
-                    const long long idx = row + jz;
-#pragma unroll
-                    for (int c = 0; c < CC; ++c)
-                        if (c < ncc) {
-                            const float2 g = __ldg(grid + (long long)c * a.coil_stride + idx);
-                            acc[c].x = fmaf(g.x, wt, acc[c].x);
-                            acc[c].y = fmaf(g.y, wt, acc[c].y);
-                        }
                 }
             }
         }
     }
-    }
     const float d = a.dcf ? a.dcf[i] : 1.f;
-    float2* out = a.yv + i * a.nch + c0;
+    a.yv[i * a.nch + c] = cscale(acc, d);
+}
+
+// ---------------------------------------------------------------------------
+// The same from the quad grid (fwd_x_quad.cuh): 4 / CPL lanes share a sample
+// and a quad of coils, CPL coils each, so a warp's load of one tap of 8 to 32
+// samples takes one 32-byte sector per sample with nothing in it but the
+// tap's coils.  Every lane adds its coils' taps in the order of k_interp
+// (x, y, z) with the same products and tests: the same bits.  Quads are the
+// fastest block index, as the coils above.  Bound by the L1's row rate (each
+// sample's sector is a row of its own): a tap of 4 coils costs one, against
+// three per coil for the 6-point rows of a coil plane.  1.32 M sample-coils
+// (one bin of 110 080 samples, 12 coils, w = 4): 296 -> 72 us.
+// ---------------------------------------------------------------------------
+
+// The 4 x 4 x 4 form of a sample (all three supports hold exactly four
+// candidates): first candidates and the factors moved to 0 .. 3.
+struct Taps4 {
+    float wx[4], wy[4], wz[4];
+    int x0, y0, z0;
+};
+CGS_D bool taps4(const float (&w)[15], Taps4& t)
+{
+    int n = 0;
+    t.x0 = w[0] == 0.f;
+    t.y0 = w[5] == 0.f;
+    t.z0 = w[10] == 0.f;
 #pragma unroll
-    for (int c = 0; c < CC; ++c)
-        if (c < ncc) out[c] = cscale(acc[c], d);
+    for (int q = 0; q < 4; ++q) {
+        t.wx[q] = t.x0 ? w[q + 1] : w[q];
+        t.wy[q] = t.y0 ? w[6 + q] : w[5 + q];
+        t.wz[q] = t.z0 ? w[11 + q] : w[10 + q];
+        n += (t.wx[q] != 0.f) + (t.wy[q] != 0.f) + (t.wz[q] != 0.f);
+    }
+    // no fifth candidate
+    return n == 12 && (t.x0 || w[4] == 0.f) && (t.y0 || w[9] == 0.f) && (t.z0 || w[14] == 0.f);
+}
+
+template <int CPL>
+struct CoilVec;
+template <>
+struct CoilVec<1> {
+    float2 c[1];
+    CGS_D void load(const float2* p) { c[0] = __ldg(p); }
+};
+template <>
+struct CoilVec<2> {
+    float2 c[2];
+    CGS_D void load(const float2* p)
+    {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+        c[0] = make_float2(v.x, v.y);
+        c[1] = make_float2(v.z, v.w);
+    }
+};
+template <>
+struct CoilVec<4> {
+    float2 c[4];
+    CGS_D void load(const float2* p)
+    {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(p)), u = __ldg(reinterpret_cast<const float4*>(p) + 1);
+        c[0] = make_float2(v.x, v.y);
+        c[1] = make_float2(v.z, v.w);
+        c[2] = make_float2(u.x, u.y);
+        c[3] = make_float2(u.z, u.w);
+    }
+};
+
+template <int CPL>
+__global__ void __launch_bounds__(128) k_interp_quad(InterpArgs a)
+{
+    constexpr int LPS = 4 / CPL;   // lanes per sample
+    const int bin = a.bin0 + blockIdx.z;
+    const long long s0 = a.bin_off[bin], s1 = a.bin_off[bin + 1];
+    const int nq = (a.nch + 3) / 4;
+    const int q = (int)(blockIdx.x % (unsigned)nq);
+    const long long blk = (long long)(blockIdx.x / (unsigned)nq) * (128 / LPS);
+    if (s0 + blk >= s1) return;
+    const long long i = s0 + blk + threadIdx.x / LPS;
+    const int sub = (int)(threadIdx.x % LPS) * CPL;   // first coil of the quad
+    const bool on = i < s1;
+    const int Gy = a.G[1], Gz = a.G[2];
+    const float2* grid = a.grid + (long long)blockIdx.z * a.grid_bs + (long long)q * a.coil_stride + sub;
+    float w[15];
+    int nx, ny, nz;
+    load_record(a.rec, on ? i : s1 - 1, w, nx, ny, nz);
+    float2 acc[CPL];
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) acc[c] = make_float2(0.f, 0.f);
+    auto add = [&](const CoilVec<CPL>& v, float wt) {
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+            acc[c].x = fmaf(v.c[c].x, wt, acc[c].x);
+            acc[c].y = fmaf(v.c[c].y, wt, acc[c].y);
+        }
+    };
+    Taps4 t;
+    if (__all_sync(0xffffffffu, taps4(w, t))) {
+        // every candidate lies in the grid: loads without a test, four rows in flight
+        const float2* g = grid + (((long long)(nx - 2 + t.x0) * Gy + (ny - 2 + t.y0)) * Gz + (nz - 2 + t.z0)) * 4;
+#pragma unroll
+        for (int ix = 0; ix < 4; ++ix) {
+            CoilVec<CPL> v[4][4];
+#pragma unroll
+            for (int iy = 0; iy < 4; ++iy)
+#pragma unroll
+                for (int iz = 0; iz < 4; ++iz) v[iy][iz].load(g + ((long long)(ix * Gy + iy) * Gz + iz) * 4);
+#pragma unroll
+            for (int iy = 0; iy < 4; ++iy) {
+                const float wxy = t.wx[ix] * t.wy[iy];
+#pragma unroll
+                for (int iz = 0; iz < 4; ++iz) {
+                    const float wt = wxy * t.wz[iz];
+                    if (wt > a.thresh) add(v[iy][iz], wt);
+                }
+            }
+        }
+    } else {
+        const float2* g = grid + (((long long)(nx - 2) * Gy + (ny - 2)) * Gz + (nz - 2)) * 4;
+#pragma unroll
+        for (int ix = 0; ix < 5; ++ix)
+#pragma unroll
+            for (int iy = 0; iy < 5; ++iy) {
+                const float wxy = w[ix] * w[5 + iy];
+                CoilVec<CPL> v[5];
+                float wt[5];
+#pragma unroll
+                for (int iz = 0; iz < 5; ++iz) {
+                    wt[iz] = wxy * w[10 + iz];   // 0 outside the support or the grid
+                    if (wt[iz] > a.thresh) v[iz].load(g + ((long long)(ix * Gy + iy) * Gz + iz) * 4);
+                }
+#pragma unroll
+                for (int iz = 0; iz < 5; ++iz)
+                    if (wt[iz] > a.thresh) add(v[iz], wt[iz]);
+            }
+    }
+    if (!on) return;
+    const float d = a.dcf ? a.dcf[i] : 1.f;
+    const int c0 = 4 * q + sub;
+#pragma unroll
+    for (int c = 0; c < CPL; ++c)
+        if (c0 + c < a.nch) a.yv[i * a.nch + c0 + c] = cscale(acc[c], d);
 }
 
 // ---------------------------------------------------------------------------

@@ -88,21 +88,19 @@ cudaError_t launch_tap_records(const double* k, const int* sample_idx, long long
     return cudaGetLastError();
 }
 
-// coils per interpolation thread: one of 2, 4, 6, 8 (autotuned per context)
+// cc: coils per thread of the quad form (1, 2 or 4; 6 and 8 count as 4); 0: 2
 cudaError_t launch_interp(const InterpArgs& a, long long max_bin_samples, int nbins, int cc, cudaStream_t s)
 {
     if (max_bin_samples == 0 || nbins == 0) return cudaSuccess;
-    const long long nblk = ((max_bin_samples + 127) / 128) * ((a.nch + cc - 1) / cc);
-    if (nblk > 0x7fffffffLL) return cudaErrorInvalidValue;
+    const int cpl = !a.quad || cc == 1 ? 1 : cc == 0 || cc == 2 ? 2 : 4;
+    const int per = a.quad ? 128 * cpl / 4 : 128, chunks = a.quad ? (a.nch + 3) / 4 : a.nch;
+    const long long nblk = ((max_bin_samples + per - 1) / per) * chunks;
+    if (nblk > 0x7fffffffLL || cc < 0 || cc > 8) return cudaErrorInvalidValue;
     dim3 grid((unsigned)nblk, 1u, (unsigned)nbins);
-    switch (cc) {
-    case 1: k_interp<1><<<grid, 128, 0, s>>>(a); break;
-    case 2: k_interp<2><<<grid, 128, 0, s>>>(a); break;
-    case 4: k_interp<4><<<grid, 128, 0, s>>>(a); break;
-    case 6: k_interp<6><<<grid, 128, 0, s>>>(a); break;
-    case 8: k_interp<8><<<grid, 128, 0, s>>>(a); break;
-    default: return cudaErrorInvalidValue;
-    }
+    if (!a.quad) k_interp<<<grid, 128, 0, s>>>(a);
+    else if (cpl == 1) k_interp_quad<1><<<grid, 128, 0, s>>>(a);
+    else if (cpl == 2) k_interp_quad<2><<<grid, 128, 0, s>>>(a);
+    else k_interp_quad<4><<<grid, 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 

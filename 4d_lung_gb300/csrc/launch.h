@@ -21,6 +21,9 @@ bool encode_strided_map(CUtensorMap* map, const StridedPassArgs& a, int A, int b
 // 3-D tensor map [nbins][L][B] of 4-byte spectrum values with a TB x
 // box_rows box; false when the buffer or pitch is not 16-byte aligned
 bool encode_spectrum_map(CUtensorMap* map, const float* P, long long B, int L, int nbins, int TB, int* box_rows);
+// 4-D map [items][1][Lin][B] with a TB x box_rows box (rows past Lin read 0)
+bool encode_items_map(CUtensorMap* map, const float2* in, int B, int Lin, long long item_stride, long long items,
+                      int TB, int box_rows, int promo);
 const int* fft_supported_list(int* n);
 // columns per tile of the strided passes of line length L (0: unsupported)
 int fft_strided_cols(int L);
@@ -30,8 +33,13 @@ int fft_strided_cols(int L);
 // strided passes' width (0: unsupported)
 int fft_listed_cols(int L, int lo, int I);
 
+// columns of a unit of the forward x pass over quads of coils, and the split
+// of the line (0: unsupported)
+int fft_quad_cols(int L, int lo, int I, int* R1, int* R2);
+
 // One launch per pass; `batch` items along blockIdx.y.
 cudaError_t launch_strided(int L, int sign, const StridedPassArgs& a, int A, int batch, cudaStream_t s);
+cudaError_t launch_fwd_x_quad(int L, const FwdXQuadArgs& a, cudaStream_t s);
 cudaError_t launch_contig(int L, int sign, const ContigPassArgs& a, int batch, cudaStream_t s);
 cudaError_t launch_fwd_z(int L, const FwdZArgs& a, int batch, cudaStream_t s);
 
@@ -58,6 +66,7 @@ cudaError_t csr_count_and_scan(const CsrBuildArgs& a, long long npts, unsigned* 
                                size_t scan_tmp_elems, unsigned long long* entries, cudaStream_t s);
 cudaError_t csr_fill_and_order(const CsrBuildArgs& a, long long npts, cudaStream_t s);
 size_t csr_scan_tmp_elems(long long n);
+cudaError_t launch_touch_mask(const TouchMaskArgs& a, cudaStream_t s);
 cudaError_t launch_spread_csr(const CsrSpreadArgs& a, bool kahan, bool staged, cudaStream_t s);
 
 // samples: reference order [nch][ns] <-> sorted, coil-interleaved [total][nch]
@@ -120,7 +129,7 @@ cudaError_t plain_dot(const float2* p, const float2* q, long long n, double* par
 // Loss gradients (grad.cu)
 cudaError_t launch_tap_grad_records(const double* k, const int* sample_idx, long long n, const KbParams& kb,
                                     TapRecord* out, cudaStream_t s);
-int interp_grad_blocks(long long n);
+int interp_grad_blocks(long long n, bool quad);
 cudaError_t launch_interp_grad(const InterpGradArgs& a, cudaStream_t s);
 cudaError_t launch_check_finite(const double* v, long long n, int* bad, cudaStream_t s);
 cudaError_t launch_pair_grad(const PairGradArgs& a, cudaStream_t s);

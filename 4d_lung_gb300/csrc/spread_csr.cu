@@ -94,6 +94,38 @@ __global__ void k_csr_order(CsrBuildArgs a, long long npts)
     }
 }
 
+// One thread per mask word: 4 k2 rows x tbq columns of one k1.
+__global__ void k_touch_mask(TouchMaskArgs a)
+{
+    const int r2w = (a.R2 + 3) / 4;
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= a.ntl * a.nsub * a.R1 * r2w) return;
+    const int w = (int)(e % r2w), k1 = (int)((e / r2w) % a.R1);
+    const long long ts = e / r2w / a.R1;
+    const int2 t = a.tiles[ts / a.nsub];
+    const int f0 = t.y + (int)(ts % a.nsub) * a.tbq;
+    const int* ct = a.col_tile + (long long)t.x * a.ncol;
+    unsigned m = 0;
+    for (int c = 0; c < a.tbq && f0 + c < a.ncol; ++c) {
+        const int J = ct[f0 + c];   // the matrix's listing holds every listed x-pass column
+        if (J < 0) continue;
+        for (int q = 0; q < 4 && 4 * w + q < a.R2; ++q) {
+            const int x = k1 + a.R1 * (4 * w + q);
+            const long long p = ((long long)J * a.Gx + x) * a.tb + (f0 + c) % a.tb;
+            if (a.ptr[p + 1] > a.ptr[p]) m |= 1u << (8 * q + c);
+        }
+    }
+    a.mask[e] = m;
+}
+
+cudaError_t launch_touch_mask(const TouchMaskArgs& a, cudaStream_t s)
+{
+    const long long n = a.ntl * a.nsub * a.R1 * ((a.R2 + 3) / 4);
+    if (n == 0) return cudaSuccess;
+    k_touch_mask<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // exclusive scan of unsigned counts (three-level block scan)
 // ---------------------------------------------------------------------------

@@ -321,7 +321,8 @@ int cgs_set_deterministic(cgs_ctx* ctx, int32_t on);
  * 8-column tile and chunk of spread_cc coils (2, 4 or 6, 0 by the coil
  * count), the grid kept in shared memory -- where the grid is not twice the
  * image along x, or the coil count has no such chunk, variant 6 runs),
- * coils per interpolation thread (1, 2, 4, 6, 8).  Variants 1, 2, 4, 5, 6,
+ * coils per interpolation thread (1, 2, 4, 6, 8; with coils in quads 6 and
+ * 8 count as 4).  Variants 1, 2, 4, 5, 6,
  * 7, 8 and every interpolation shape give bitwise-identical results. */
 int cgs_set_launch_shape(cgs_ctx* ctx, int32_t spread_cc, int32_t spread_variant, int32_t interp_cc);
 

@@ -1,0 +1,46 @@
+"""The forward grid in quads of coils (three coils or more) against coil
+planes (one coil): every coil goes through the same operations in the same
+order in either form, so the samples must agree bit for bit.  Sizes at the
+edges of the quad x pass: one padded and one full quad, image lines in one and
+two copies, 4- and 8-column units, half-pruned lines and general ones."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    ((16, 16, 12), (32, 32, 24), 3, 4.0),      # the smallest line, 3 of 4 coils
+    ((32, 24, 20), (64, 48, 40), 4, 4.25),     # 5 candidates on some axes
+    ((33, 17, 13), (64, 32, 24), 5, 4.0),      # odd image, a quad of one coil
+    ((75, 16, 12), (128, 32, 24), 9, 4.25),    # general line, three quads
+    ((128, 16, 12), (256, 32, 24), 4, 4.0),    # half-pruned, 8-column units
+    ((160, 16, 12), (320, 32, 24), 6, 4.0),    # half-pruned, 4-column units
+    ((300, 16, 12), (320, 32, 24), 3, 4.0),    # input rows in two copies
+    ((88, 16, 12), (176, 32, 24), 4, 4.0),     # R2 odd
+    ((176, 16, 12), (352, 32, 24), 3, 4.0),    # R1 = 32
+]
+
+
+@pytest.mark.parametrize("img,grid,nch,kb_w", CASES)
+@pytest.mark.parametrize("pruned", [True, False])
+def test_quads_equal_coil_planes_bitwise(gpu_lib, cgs, img, grid, nch, kb_w, pruned):
+    rng = np.random.default_rng(5)
+    # a cluster of samples, some at the faces of the grid
+    k = np.concatenate([0.5 + 0.2 * rng.standard_normal((700, 3)).clip(-2, 2), rng.uniform(0, 1, (100, 3))])
+    k[:6] = [[0, 0, 0], [1, 1, 1], [0, 1, 0.5], [1, 0, 0.5], [0.5, 0, 1], [0.5, 1, 0]]
+    x = (rng.standard_normal((nch,) + img) + 1j * rng.standard_normal((nch,) + img)).astype(np.complex64)
+    kw = dict(kb_w=kb_w, kb_b=9.0)
+    r = cgs.Reco(img, grid, nch, **kw)
+    r.set_trajectory(k)
+    r.set_support_pruning(pruned)
+    one = cgs.Reco(img, grid, 1, **kw)
+    one.set_trajectory(k)
+    one.set_support_pruning(pruned)
+    y = r.nufft_fwd(x)
+    assert np.isfinite(y).all() and np.abs(y).max() > 0
+    for c in range(nch):
+        assert np.array_equal(y[c], one.nufft_fwd(x[c:c + 1])[0]), c
+    # every coils-per-thread form
+    for cc in (1, 2, 4):
+        r.set_launch_shape(0, 8, cc)
+        assert np.array_equal(r.nufft_fwd(x), y), cc
