@@ -39,6 +39,10 @@ struct QuadLayout {
     static constexpr int RM = R1 > R2 ? R1 : R2;
     static constexpr int W = 4 * TBQ;            // exchange row: coils x columns
     static constexpr int NT = W * RM;
+    // resident blocks asked of the compiler: 64 to 102 registers a thread (two
+    // of L = 320's blocks per SM instead of one: 1.31 -> 0.77 ms, 16 coils of
+    // a 320 x 320 x 224 grid)
+    static constexpr int MINB = RM <= 16 ? (NT <= 256 ? 3 : 2) : RM <= 24 ? 2 : 1;
     static constexpr int R2W = (R2 + 3) / 4;     // mask words of a row group k1
     // the x rows of one coil, rounded up to 128 bytes
     __host__ __device__ static int coil_elems(int rows) { return (rows * TBQ + 15) & ~15; }
@@ -57,7 +61,7 @@ struct QuadLayout {
 
 template <int R1, int R2, int TBQ, int MODE>
 __global__ void __launch_bounds__(QuadLayout<R1, R2, TBQ>::NT,
-                                  QuadLayout<R1, R2, TBQ>::RM > 16 ? 1 : (QuadLayout<R1, R2, TBQ>::NT <= 256 ? 3 : 2))
+                                  QuadLayout<R1, R2, TBQ>::MINB)
 k_fwd_x_quad(FwdXQuadArgs a, const __grid_constant__ CUtensorMap tmap, int nunits, int per_quad, int nsub,
              int box_rows, int nbox)
 {

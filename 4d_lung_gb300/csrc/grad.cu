@@ -163,9 +163,10 @@ __global__ void __launch_bounds__(128) k_interp_grad(InterpGradArgs a)
 // 32-byte sector per sample.  A lane adds its coil's value and derivatives
 // over the taps in the order of the kernels above with the same products and
 // tests, and the coil sums run in coil order: the same bits.  1 572 864
-// samples, 12 coils: k_interp_grad 7.93 -> 3.31 ms (its multiply-adds and the
-// weights formed anew per quad bound it now); 262 144 samples in four bins, 8
-// coils: k_pair_grad 0.36 -> 0.11 ms a launch.
+// samples, 12 coils: k_interp_grad 7.93 -> 3.31 ms, 2.4 ms with seven blocks
+// per SM (six and eight, which spills 1.4 KB: 2.5 and 2.8); its multiply-adds
+// and the weights formed anew per quad bound it now.  262 144 samples in four
+// bins, 8 coils: k_pair_grad 0.36 -> 0.11 ms a launch.
 // ---------------------------------------------------------------------------
 struct GradSums {
     float2 y, d0, d1, d2;
@@ -271,7 +272,7 @@ CGS_D GradSums quad_grad_sums(const float2* __restrict__ g, const QuadTaps& t, i
 
 constexpr int QG_SAMPLES = 32;   // samples per block of 128 threads
 
-__global__ void __launch_bounds__(4 * QG_SAMPLES) k_interp_grad_quad(InterpGradArgs a)
+__global__ void __launch_bounds__(4 * QG_SAMPLES, 7) k_interp_grad_quad(InterpGradArgs a)
 {
     __shared__ double s_red[QG_SAMPLES / 8];
     const int lane = threadIdx.x & 31, sub = threadIdx.x & 3, lead = lane & ~3;
@@ -435,7 +436,7 @@ __global__ void __launch_bounds__(128) k_pair_grad(PairGradArgs a)
     }
 }
 
-__global__ void __launch_bounds__(4 * QG_SAMPLES) k_pair_grad_quad(PairGradArgs a)
+__global__ void __launch_bounds__(4 * QG_SAMPLES, 6) k_pair_grad_quad(PairGradArgs a)
 {
     const int lane = threadIdx.x & 31, sub = threadIdx.x & 3, lead = lane & ~3;
     const long long j = (long long)blockIdx.x * QG_SAMPLES + threadIdx.x / 4;

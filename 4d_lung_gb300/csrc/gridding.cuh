@@ -184,7 +184,9 @@ __global__ void __launch_bounds__(128) k_interp(InterpArgs a)
 // fastest block index, as the coils above.  Bound by the L1's row rate (each
 // sample's sector is a row of its own): a tap of 4 coils costs one, against
 // three per coil for the 6-point rows of a coil plane.  1.32 M sample-coils
-// (one bin of 110 080 samples, 12 coils, w = 4): 296 -> 72 us.
+// (one bin of 110 080 samples, 12 coils, w = 4): 296 -> 72 us, 65 with eight
+// blocks per SM; ten or twelve leave too few registers for the loads in flight
+// (106 and 116).
 // ---------------------------------------------------------------------------
 
 // The 4 x 4 x 4 form of a sample (all three supports hold exactly four
@@ -241,7 +243,7 @@ struct CoilVec<4> {
 };
 
 template <int CPL>
-__global__ void __launch_bounds__(128) k_interp_quad(InterpArgs a)
+__global__ void __launch_bounds__(128, 8) k_interp_quad(InterpArgs a)
 {
     constexpr int LPS = 4 / CPL;   // lanes per sample
     const int bin = a.bin0 + blockIdx.z;
