@@ -63,6 +63,23 @@ void use_trajectory(cgs_ctx* c, const torch::Tensor& k)
     s.serial = cgs_trajectory_serial(c);
 }
 
+// A backward pass unpacks its own tensor object for the k that its forward
+// pass saved, so the test above would not know it.  The forward pass notes the
+// context's trajectory serial number after its upload: while that is still
+// the context's, the coordinates on it are the saved ones (autograd refuses a
+// saved tensor that was modified in place), and only another trajectory set in
+// between makes the backward pass upload its k again.  (An unrolled CG of 3
+// iterations over 262 144 samples uploaded one k 13 times and rebuilt its
+// lists 6 times.)
+void note_trajectory(AutogradContext* ctx, cgs_ctx* c)
+{
+    ctx->saved_data["k_serial"] = (int64_t)cgs_trajectory_serial(c);
+}
+void use_saved_trajectory(AutogradContext* ctx, cgs_ctx* c, const torch::Tensor& k)
+{
+    if (ctx->saved_data["k_serial"].toInt() != (int64_t)cgs_trajectory_serial(c)) use_trajectory(c, k);
+}
+
 // Orders the library's work after PyTorch's pending work on the current
 // stream and PyTorch's later work after the library's: an event on each
 // side (the context keeps its own stream and its captured graphs).
@@ -155,6 +172,7 @@ struct ApplyA : public torch::autograd::Function<ApplyA> {
         check(c, cgs_apply_ehde_d(c, (int32_t)bin0, (int32_t)nb, reinterpret_cast<const float*>(p.data_ptr()),
                                   reinterpret_cast<float*>(q.data_ptr())),
               "cgs_apply_ehde_d");
+        note_trajectory(ctx, c);
         ctx->save_for_backward({p, k});
         ctx->saved_data["handle"] = handle;
         ctx->saved_data["bin0"] = bin0;
@@ -175,7 +193,7 @@ struct ApplyA : public torch::autograd::Function<ApplyA> {
         if (ctx->needs_input_grad(1)) gk = torch::zeros({k.size(0), 3}, k.options().dtype(torch::kFloat32));
         {
             StreamJoin join(c, v);   // PyTorch's later work (the conversion below) waits for these
-            use_trajectory(c, k);
+            use_saved_trajectory(ctx, c, k);
             if (gp.defined())
                 check(c, cgs_apply_ehde_d(c, bin0, nb, reinterpret_cast<const float*>(v.data_ptr()),
                                           reinterpret_cast<float*>(gp.data_ptr())),
@@ -200,6 +218,7 @@ struct Rhs : public torch::autograd::Function<Rhs> {
         StreamJoin join(c, y);
         use_trajectory(c, k);
         check(c, cgs_rhs_d(c, (int32_t)bin0, (int32_t)nb, y.data_ptr(), b.data_ptr()), "cgs_rhs_d");
+        note_trajectory(ctx, c);
         ctx->save_for_backward({y, k});
         ctx->saved_data["handle"] = handle;
         ctx->saved_data["bin0"] = bin0;
@@ -218,7 +237,7 @@ struct Rhs : public torch::autograd::Function<Rhs> {
         if (ctx->needs_input_grad(1)) {   // tensor inputs: y is 0, k is 1
             gk = torch::zeros({k.size(0), 3}, k.options().dtype(torch::kFloat32));
             StreamJoin join(c, v);   // ends before the conversion below
-            use_trajectory(c, k);
+            use_saved_trajectory(ctx, c, k);
             check(c, cgs_rhs_vjp_k_d(c, bin0, nb, y.data_ptr(), v.data_ptr(), gk.data_ptr()), "cgs_rhs_vjp_k_d");
         }
         return {torch::Tensor(), torch::Tensor(), torch::Tensor(), torch::Tensor(),
