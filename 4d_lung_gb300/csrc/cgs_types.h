@@ -143,11 +143,25 @@ struct TapRecord {
     float4 q[4];   // w[0..14] = x(5) y(5) z(5); q[3].w holds the packed nearest point
 };
 
+// A power series with positive terms, sum_k c_k s^k on 0 <= s <= 1: the first
+// nd coefficients as float pairs (hi + lo), the rest (together below 2^-30 of
+// the sum) as floats.
+constexpr int KB_ND = 26, KB_NF = 16;
+struct KbSeries {
+    int nd, nf;        // nd 0: not available (a shape beyond the arrays)
+    float2 cd[KB_ND];
+    float cf[KB_NF];
+};
+
 struct KbParams {
     int G[3];          // grid size
     float w;           // KB width (cells)
     float b;           // KB shape
     float thresh;      // absolute tap threshold
+    KbSeries i0;       // I0(b sqrt(s))
+    KbSeries i1;       // I1(b sqrt(s)) / sqrt(s)
+    float2 rC[3];      // per axis 1 / C, C = 100 w dk, as a float pair
+    float2 f0[3];      // per axis b * 2 / (w dk) / C, as a float pair
 };
 
 struct InterpArgs {

@@ -23,7 +23,7 @@ namespace cgs {
 // float index * float dk, distance rounded to float).  For
 // f = I0(b s) / C, s = sqrt(1 - q^2), q = 2 |d| / (w dk):
 //   df/dk = -(I1(b s) / s) * b * q * sign(d) * 2 / (w dk) / C,
-// with I1(b s) / s -> b / 2 as s -> 0.
+// with I1(b s) / s -> b / 2 as s -> 0; its power series in s^2 (kb_series).
 __global__ void k_tap_grad_records(const double* __restrict__ k, const int* __restrict__ sample_idx, long long n,
                                    KbParams kb, TapRecord* __restrict__ out)
 {
@@ -49,13 +49,19 @@ __global__ void k_tap_grad_records(const double* __restrict__ k, const int* __re
                 const float d = (float)fabs(dd);
                 if (!(d > wHalf * dk)) {
                     const float q = (float)(2.f * d) / (float)(kb.w * dk);
-                    const double s2 = __dadd_rn(1.0, -__dmul_rn((double)q, (double)q));
-                    const double s = s2 > 0.0 ? sqrt(s2) : 0.0;
-                    const double b = (double)kb.b;
-                    const double i1s = s > 1e-12 ? cyl_bessel_i1(b * s) / s : 0.5 * b;
-                    const double C = (double)(float)(100.0f * kb.w * dk);
-                    const double dv = -i1s * b * (double)q * (2.0 / ((double)kb.w * (double)dk)) / C;
-                    val = (float)(dd >= 0.0 ? dv : -dv);
+                    float dv;
+                    if (kb.i1.nd > 0) {
+                        const float2 f = pair_mul(make_float2(q, 0.f), kb.f0[a]);
+                        dv = -pair_mul(kb_series(kb.i1, pair_one_minus_sq(q)), f).x;
+                    } else {
+                        const double s2 = __dadd_rn(1.0, -__dmul_rn((double)q, (double)q));
+                        const double s = s2 > 0.0 ? sqrt(s2) : 0.0;
+                        const double b = (double)kb.b;
+                        const double i1s = s > 1e-12 ? cyl_bessel_i1(b * s) / s : 0.5 * b;
+                        const double C = (double)(float)(100.0f * kb.w * dk);
+                        dv = (float)(-i1s * b * (double)q * (2.0 / ((double)kb.w * (double)dk)) / C);
+                    }
+                    val = dd >= 0.0 ? dv : -dv;
                 }
             }
             f[a * TAPS_1D + j] = val;
@@ -331,6 +337,31 @@ cudaError_t launch_interp_grad(const InterpGradArgs& a, cudaStream_t s)
 {
     if (a.quad) k_interp_grad_quad<<<(unsigned)interp_grad_blocks(a.n, true), 4 * QG_SAMPLES, 0, s>>>(a);
     else k_interp_grad<2><<<(unsigned)interp_grad_blocks(a.n, false), 128, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+// Sum of the loss partials in one block, in a fixed order: one value to copy
+// back instead of all of them.
+__global__ void __launch_bounds__(1024) k_loss_sum(double* partials, int n)
+{
+    __shared__ double s[32];
+    double v = 0.0;
+    for (int i = threadIdx.x; i < n; i += 1024) v += partials[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        v = s[threadIdx.x];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (threadIdx.x == 0) partials[0] = v;
+    }
+}
+
+cudaError_t launch_loss_sum(double* partials, int n, cudaStream_t s)
+{
+    k_loss_sum<<<1, 1024, 0, s>>>(partials, n);
     return cudaGetLastError();
 }
 

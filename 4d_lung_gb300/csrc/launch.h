@@ -131,6 +131,8 @@ cudaError_t launch_tap_grad_records(const double* k, const int* sample_idx, long
                                     TapRecord* out, cudaStream_t s);
 int interp_grad_blocks(long long n, bool quad);
 cudaError_t launch_interp_grad(const InterpGradArgs& a, cudaStream_t s);
+// partials[0] = the sum of the n partials
+cudaError_t launch_loss_sum(double* partials, int n, cudaStream_t s);
 cudaError_t launch_check_finite(const double* v, long long n, int* bad, cudaStream_t s);
 cudaError_t launch_pair_grad(const PairGradArgs& a, cudaStream_t s);
 cudaError_t launch_pm_init(float* w, float2* v, long long n, cudaStream_t s);
