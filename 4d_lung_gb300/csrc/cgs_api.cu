@@ -177,6 +177,8 @@ struct cgs_ctx {
     // workspace
     int ws_bins = 0;
     DevBuf d_zbuf, d_ybuf, d_grid, d_yv, d_img, d_data;
+    // density weights (cgs_pipe_menon_dcf)
+    DevBuf d_pm_w, d_pm_max, d_pm_owner, d_pm_out;
     // CG
     DevBuf d_b, d_x, d_r, d_pv, d_q, d_state, d_partials, d_partials2, d_res;
     // while a fused solve is recorded: the vectors whose pending updates the
@@ -2792,13 +2794,46 @@ int cgs_pipe_menon_dcf(cgs_ctx* c, int32_t iters, float* dcf, int32_t on_device)
     CGS_TRY(check_ready(c, false));
     if (!dcf || iters < 1 || iters > 1000) return fail(c, CGS_ERR_ARG, "bad arguments");
     const long long n = c->total;
-    DevBuf w, v, u;
+    const bool csr = c->sup_built && c->csr_valid;
+    DevBuf& w = c->d_pm_w;
+    DevBuf v, u;   // complex values of the tiled kernels
     CGS_CUDA(c, w.ensure(std::max<long long>(n, 1) * sizeof(float)));
-    CGS_CUDA(c, v.ensure(std::max<long long>(n, 1) * sizeof(float2)));
-    CGS_CUDA(c, u.ensure(std::max<long long>(n, 1) * sizeof(float2)));
+    if (!csr) {
+        CGS_CUDA(c, v.ensure(std::max<long long>(n, 1) * sizeof(float2)));
+        CGS_CUDA(c, u.ensure(std::max<long long>(n, 1) * sizeof(float2)));
+    }
     CGS_CUDA(c, launch_pm_init(w.as<float>(), v.as<float2>(), n, c->stream));
+    // over the transposed tap matrix: as many bins at once as the workspace
+    // holds real grids
+    const int per = (int)std::min<long long>(2 * c->ws_bins * (fwd_grid_elems(c) / c->Ng), 65535);
+    for (int it = 0; csr && it < iters; ++it)
+        for (int g = 0; g < c->nbins; g += per) {
+            const int nb = std::min(per, c->nbins - g);
+            const bool xl = c->csr_list == 1;
+            const std::vector<long long>& off = xl ? c->h_sup_off : c->h_spr_off;
+            PmArgs pa{};
+            pa.ptr = c->d_csr_ptr.as<unsigned>();
+            pa.ent = c->d_csr_ent.as<int2>();
+            pa.tiles = (xl ? c->d_sup_tiles : c->d_spr_tiles).as<int2>();
+            pa.j0 = off[g];
+            pa.nj = off[g + nb] - off[g];
+            pa.tb = xl ? c->sup_tb : c->spr_tb;
+            for (int a = 0; a < 3; ++a) pa.G[a] = c->G[a];
+            pa.Ng = c->Ng;
+            pa.bin0 = g;
+            pa.nbins = nb;
+            pa.rec = c->d_rec.as<TapRecord>();
+            pa.bin_off = c->d_bin_off.as<long long>();
+            pa.thresh = c->thresh;
+            pa.grid = c->d_grid.as<float>();
+            pa.w = w.as<float>();
+            long long mx = 0;
+            for (int b = g; b < g + nb; ++b) mx = std::max(mx, c->h_bin_off[b + 1] - c->h_bin_off[b]);
+            CGS_LAUNCH(c, launch_pm_step(pa, mx, c->stream));
+            ++c->launches;   // spreading, interpolation with the update
+        }
     const long long grid_bs = c->Ng;   // one "coil" per bin
-    for (int it = 0; it < iters; ++it) {
+    for (int it = 0; !csr && it < iters; ++it) {
         for (int g = 0; g < c->nbins; g += c->ws_bins * c->nch) {
             // the workspace holds ws_bins * nch grids: as many single-coil bins at once
             const int nb = std::min(c->ws_bins * c->nch, c->nbins - g);
@@ -2842,22 +2877,15 @@ int cgs_pipe_menon_dcf(cgs_ctx* c, int32_t iters, float* dcf, int32_t on_device)
         CGS_CUDA(c, launch_pm_update(w.as<float>(), v.as<float2>(), u.as<float2>(), n, c->stream));
     }
     // per-bin normalisation by the maximum, scatter to the reference's order
-    std::vector<float> hw(std::max<long long>(n, 1));
-    std::vector<int> hs(std::max<long long>(n, 1));
-    CGS_CUDA(c, cudaMemcpyAsync(hw.data(), w.p, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-    CGS_CUDA(c, cudaMemcpyAsync(hs.data(), c->d_sorted.p, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CGS_CUDA(c, cudaStreamSynchronize(c->stream));
-    std::vector<float> out(c->ns, 0.f);
-    for (int b = 0; b < c->nbins; ++b) {
-        float mx = 0.f;
-        for (long long j = c->h_bin_off[b]; j < c->h_bin_off[b + 1]; ++j) mx = std::max(mx, hw[j]);
-        const float inv = mx > 0.f ? 1.f / mx : 0.f;
-        for (long long j = c->h_bin_off[b]; j < c->h_bin_off[b + 1]; ++j) out[hs[j]] = hw[j] * inv;
-    }
-    if (on_device)
-        CGS_CUDA(c, cudaMemcpyAsync(dcf, out.data(), (size_t)c->ns * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-    else
-        std::copy(out.begin(), out.end(), dcf);
+    DevBuf &mx = c->d_pm_max, &owner = c->d_pm_owner, &out = c->d_pm_out;
+    CGS_CUDA(c, mx.ensure((size_t)c->nbins * sizeof(unsigned)));
+    CGS_CUDA(c, owner.ensure((size_t)c->ns * sizeof(int)));
+    if (!on_device) CGS_CUDA(c, out.ensure((size_t)c->ns * sizeof(float)));
+    float* dst = on_device ? dcf : out.as<float>();
+    CGS_LAUNCH(c, launch_pm_finish(w.as<float>(), c->d_sorted.as<int>(), c->d_bin_off.as<long long>(), c->nbins,
+                                 c->max_bin, c->ns, mx.as<unsigned>(), owner.as<int>(), dst, c->stream));
+    if (!on_device)
+        CGS_CUDA(c, cudaMemcpyAsync(dcf, dst, (size_t)c->ns * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
     CGS_CUDA(c, cudaStreamSynchronize(c->stream));
     return check_timeout(c);
 }

@@ -307,6 +307,24 @@ struct PsfSpreadArgs {
     double* out;               // [nf0][nf1][nf2]
 };
 
+// Iterative density weights over the transposed tap matrix (grad.cu): the
+// bins [bin0, bin0 + nbins) with one real grid each.
+struct PmArgs {
+    const unsigned* ptr;       // matrix of the listing below (CsrSpreadArgs)
+    const int2* ent;
+    const int2* tiles;
+    long long j0, nj;
+    int tb;
+    int G[3];
+    long long Ng;
+    int bin0, nbins;
+    const TapRecord* rec;
+    const long long* bin_off;
+    float thresh;
+    float* grid;               // [nbins][Ng]
+    float* w;                  // [total samples]
+};
+
 // Loss gradient pass (grad.cu): one bin's samples [s0, s0 + n) in sorted order.
 struct InterpGradArgs {
     const float2* grid;        // one bin's grid, as in InterpArgs

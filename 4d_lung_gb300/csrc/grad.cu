@@ -565,13 +565,145 @@ __global__ void k_pm_init(float* __restrict__ w, float2* __restrict__ v, long lo
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     w[i] = 1.f;
-    v[i] = make_float2(1.f, 0.f);
+    if (v) v[i] = make_float2(1.f, 0.f);
 }
 
 cudaError_t launch_pm_init(float* w, float2* v, long long n, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
     k_pm_init<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w, v, n);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// The same iteration over the transposed tap matrix.  The values are real, so
+// the grid is one float a point; the spreading is a gather of each touched
+// point's row (no other point is read), the interpolation ends with the
+// update.  Sums run in the order of k_spread and k_interp with the same fused
+// multiply-adds: the same weights bit for bit.  16 bins, 1 572 864 samples,
+// grid 256 x 256 x 192, an iteration: k_spread 1.46 + k_interp 0.18 ms against
+// 0.66 + 0.20 (the rows' scattered reads bound the gather).
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) k_pm_spread(PmArgs a)
+{
+    const int pts = a.G[0] * a.tb;
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= a.nj * pts) return;
+    const unsigned* p = a.ptr + a.j0 * pts + e;
+    unsigned q = __ldg(p);
+    const unsigned e1 = __ldg(p + 1);
+    if (q == e1) return;
+    float acc = 0.f;
+    for (; q + 1 < e1; q += 2) {   // four or eight taps in flight: 0.83 ms
+        const int2 u = __ldg(a.ent + q), v = __ldg(a.ent + q + 1);
+        const float wu = __ldg(a.w + u.x), wv = __ldg(a.w + v.x);
+        acc = fmaf(wu, __int_as_float(u.y), acc);
+        acc = fmaf(wv, __int_as_float(v.y), acc);
+    }
+    if (q < e1) {
+        const int2 u = __ldg(a.ent + q);
+        acc = fmaf(__ldg(a.w + u.x), __int_as_float(u.y), acc);
+    }
+    const long long j = e / pts;
+    const int i = (int)(e - j * pts), x = i / a.tb;
+    const int2 t = a.tiles[a.j0 + j];
+    a.grid[(long long)(t.x - a.bin0) * a.Ng + (long long)x * a.G[1] * a.G[2] + t.y + (i - x * a.tb)] = acc;
+}
+
+// One thread per sample; rows away from the ends of the grid are read as two
+// aligned 16-byte loads (8 points from the multiple of 4 at or below the row).
+__global__ void __launch_bounds__(128) k_pm_interp(PmArgs a)
+{
+    const int bin = a.bin0 + blockIdx.y;
+    const long long s0 = a.bin_off[bin], s1 = a.bin_off[bin + 1];
+    const long long i = s0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= s1) return;
+    const float* grid = a.grid + (long long)blockIdx.y * a.Ng;   // Ng is a multiple of 4
+    float w[15];
+    int nx, ny, nz;
+    load_record(a.rec, i, w, nx, ny, nz);
+    const int Gy = a.G[1], Gz = a.G[2];
+    float acc = 0.f;
+#pragma unroll
+    for (int jx = 0; jx < 5; ++jx) {
+        const float wx = w[jx];
+        if (wx == 0.f) continue;
+#pragma unroll
+        for (int jy = 0; jy < 5; ++jy) {
+            const float wxy = wx * w[5 + jy];
+            if (wxy == 0.f) continue;
+            const long long row = ((long long)(nx - 2 + jx) * Gy + (ny - 2 + jy)) * Gz + (nz - 2);
+            const long long r0 = row & ~3LL;
+            float v[8];
+            const bool vec = row >= 0 && r0 + 8 <= a.Ng;
+            const int sh = vec ? (int)(row - r0) : 0;
+            if (vec) {
+                const float4 u0 = __ldg(reinterpret_cast<const float4*>(grid + r0));
+                const float4 u1 = __ldg(reinterpret_cast<const float4*>(grid + r0) + 1);
+                v[0] = u0.x; v[1] = u0.y; v[2] = u0.z; v[3] = u0.w;
+                v[4] = u1.x; v[5] = u1.y; v[6] = u1.z; v[7] = u1.w;
+            }
+#pragma unroll
+            for (int jz = 0; jz < 5; ++jz) {
+                const float wz = w[10 + jz];
+                const float wt = wxy * wz;
+                if (wz != 0.f && wt > a.thresh) {
+                    const float g = vec ? (sh == 0 ? v[jz] : sh == 1 ? v[jz + 1] : sh == 2 ? v[jz + 2] : v[jz + 3])
+                                        : __ldg(grid + row + jz);
+                    acc = fmaf(g, wt, acc);
+                }
+            }
+        }
+    }
+    a.w[i] = acc > 0.f ? a.w[i] / acc : 0.f;
+}
+
+cudaError_t launch_pm_step(const PmArgs& a, long long max_bin, cudaStream_t s)
+{
+    const long long np = a.nj * a.G[0] * a.tb;
+    if (np > 0) k_pm_spread<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(a);
+    if (max_bin > 0) k_pm_interp<<<dim3((unsigned)((max_bin + 127) / 128), (unsigned)a.nbins), 128, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+// per bin the largest weight (weights are not negative: ordered as integers),
+// and the last bin that holds each sample
+__global__ void __launch_bounds__(256) k_pm_max(const float* __restrict__ w, const int* __restrict__ sorted,
+                                                const long long* __restrict__ bin_off, unsigned* mx, int* owner)
+{
+    const int bin = blockIdx.y;
+    unsigned m = 0;
+    for (long long i = bin_off[bin] + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < bin_off[bin + 1];
+         i += (long long)gridDim.x * blockDim.x) {
+        m = max(m, __float_as_uint(w[i]));
+        atomicMax(owner + sorted[i], bin + 1);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(mx + bin, m);
+}
+
+__global__ void __launch_bounds__(256) k_pm_scatter(const float* __restrict__ w, const int* __restrict__ sorted,
+                                                    const long long* __restrict__ bin_off, const unsigned* mx,
+                                                    const int* owner, float* __restrict__ out)
+{
+    const int bin = blockIdx.y;
+    const float m = __uint_as_float(mx[bin]);
+    const float inv = m > 0.f ? 1.f / m : 0.f;
+    for (long long i = bin_off[bin] + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < bin_off[bin + 1];
+         i += (long long)gridDim.x * blockDim.x)
+        if (owner[sorted[i]] == bin + 1) out[sorted[i]] = w[i] * inv;
+}
+
+cudaError_t launch_pm_finish(const float* w, const int* sorted, const long long* bin_off, int nbins, long long max_bin,
+                             long long ns, unsigned* mx, int* owner, float* out, cudaStream_t s)
+{
+    cudaError_t e = cudaMemsetAsync(mx, 0, (size_t)nbins * sizeof(unsigned), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(owner, 0, (size_t)ns * sizeof(int), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(out, 0, (size_t)ns * sizeof(float), s);
+    if (e != cudaSuccess || max_bin == 0) return e;
+    const dim3 grid((unsigned)std::min<long long>((max_bin + 255) / 256, 1024), (unsigned)nbins);
+    k_pm_max<<<grid, 256, 0, s>>>(w, sorted, bin_off, mx, owner);
+    k_pm_scatter<<<grid, 256, 0, s>>>(w, sorted, bin_off, mx, owner, out);
     return cudaGetLastError();
 }
 

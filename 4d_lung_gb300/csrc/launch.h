@@ -135,6 +135,12 @@ cudaError_t launch_interp_grad(const InterpGradArgs& a, cudaStream_t s);
 cudaError_t launch_loss_sum(double* partials, int n, cudaStream_t s);
 cudaError_t launch_check_finite(const double* v, long long n, int* bad, cudaStream_t s);
 cudaError_t launch_pair_grad(const PairGradArgs& a, cudaStream_t s);
+// one iteration w <- w / (C w) of the bins of a; max_bin: their longest bin
+cudaError_t launch_pm_step(const PmArgs& a, long long max_bin, cudaStream_t s);
+// out[ns] (zeroed here) = the weights over each bin's maximum, by global index;
+// a sample in several bins gets the last one's.  mx [nbins], owner [ns]: scratch
+cudaError_t launch_pm_finish(const float* w, const int* sorted, const long long* bin_off, int nbins, long long max_bin,
+                             long long ns, unsigned* mx, int* owner, float* out, cudaStream_t s);
 cudaError_t launch_pm_init(float* w, float2* v, long long n, cudaStream_t s);
 cudaError_t launch_pm_update(float* w, float2* v, const float2* u, long long n, cudaStream_t s);
 
