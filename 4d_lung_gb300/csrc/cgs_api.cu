@@ -108,10 +108,12 @@ struct cgs_ctx {
     // launch shapes (cgs_autotune): coils per spreading block (0: as many as
     // fit), coils per interpolation thread (0: 2)
     int spread_cc = 0;
-    int spread_wpp = 8;          // spreading variant: warps per x plane 1 / 2, 3 atomics, 4 / 5 pipelined,
-                                 // 6 / 7 gather over the transposed tap matrix, staged in shared memory /
-                                 // read from global memory (2 when it is not built), 8 the staged gather
-                                 // fused with the adjoint x pass (6 where that does not apply)
+    int spread_wpp = 0;          // spreading variant: warps per x plane 1 / 2, 3 atomics, 4 / 5 pipelined,
+                                 // 6 the gather over the sliced tap matrix into the quad grid (one or two
+                                 // coils: over the rows staged in shared memory), 7 the rows read from
+                                 // global memory, 8 the staged gather fused with the adjoint x pass (6 where
+                                 // that does not apply); 6 to 8 are 2 when the matrix is not built.  0: 6
+                                 // with the quad grid (quad_spread), else 8
     bool deterministic = true;   // fixed summation order everywhere (cgs_set_deterministic)
     bool spread_fused = false;   // the last adjoint half ran the fused spreading + x pass
     int interp_cc = 0;
@@ -141,13 +143,15 @@ struct cgs_ctx {
     std::vector<long long> h_spr_off;
     std::vector<int2> h_spr_tiles;
     DevBuf d_spr_tiles;
-    int csr_list = -1;                       // listing of the transposed tap matrix: 0 the spreading's,
-                                             // 1 the x passes' (fused variant 8); -1 not built
+    int csr_list = -1;                       // form of the transposed tap matrix: 0 rows over the spreading's
+                                             // listing, 1 rows over the x passes' (fused variant 8), 2 slices
+                                             // over the x passes' (quad grid); -1 not built
     // transposed tap matrix of the listed tiles' points (spreading variant 6)
     bool csr_valid = false;
     long long csr_pts = 0;
     unsigned long long csr_entries = 0;
     DevBuf d_col_tile, d_csr_cnt, d_csr_ptr, d_csr_ent, d_csr_tmp;
+    DevBuf d_sl_ord, d_sl_head, d_sl_mask, d_sl_ent, d_sl_off;   // the slices (SliceArgs; in place of d_csr_ent)
     std::vector<long long> h_live_off;       // per bin: first entry in d_live (spreading tiles)
     DevBuf d_sup_tiles, d_live, d_live_off;
     // The adjoint x pass writes its own y buffer (d_ybuf_adj), and with
@@ -490,7 +494,7 @@ int upload(cgs_ctx* c, DevBuf& b, const void* h, size_t bytes)
 
 // The transposed tap matrix over the points of the listed tiles of the
 // spreading gather (list 0, variants 6 and 7) or of the x passes (list 1,
-// the gather fused with the adjoint x pass), from the current tap records
+// the gather fused with the adjoint x pass; list 2, in slices), from the current tap records
 // and support lists.  Skipped (the gather variants then fall back to the
 // tiled kernel) when the counts could overflow 32-bit offsets.
 int build_csr(cgs_ctx* c, int list)
@@ -499,9 +503,9 @@ int build_csr(cgs_ctx* c, int list)
     c->csr_list = -1;
     c->csr_entries = 0;
     if (!c->sup_built || c->total == 0) return CGS_OK;
-    const int tbx = list == 1 ? c->sup_tb : c->spr_tb;
-    const std::vector<long long>& off = list == 1 ? c->h_sup_off : c->h_spr_off;
-    const std::vector<int2>& tl = list == 1 ? c->h_sup_tiles : c->h_spr_tiles;
+    const int tbx = list >= 1 ? c->sup_tb : c->spr_tb;
+    const std::vector<long long>& off = list >= 1 ? c->h_sup_off : c->h_spr_off;
+    const std::vector<int2>& tl = list >= 1 ? c->h_sup_tiles : c->h_spr_tiles;
     const long long ncol = (long long)c->G[1] * c->G[2];
     const long long ntl = off[c->nbins];
     const long long npts = ntl * c->G[0] * tbx;
@@ -536,10 +540,36 @@ int build_csr(cgs_ctx* c, int list)
     CGS_CUDA(c, c->d_csr_ent.ensure((ne + 2) * sizeof(int2)));
     a.ent = c->d_csr_ent.as<int2>();
     CGS_CUDA(c, csr_fill_and_order(a, npts, c->stream));
+    if (list == 2) {
+        SliceArgs sl{};
+        fft_quad_cols(c->G[0], c->lo[0], c->I[0], &sl.R1, &sl.R2);
+        sl.ptr = a.ptr;
+        sl.ent = a.ent;
+        sl.ntl = ntl;
+        sl.tb = tbx;
+        sl.pts = c->G[0] * tbx;
+        sl.head_words = slice_head_words(sl.pts);
+        const long long nsl = ntl * (sl.pts / 32);
+        CGS_CUDA(c, c->d_sl_off.ensure((size_t)(nsl + 1) * sizeof(unsigned)));
+        CGS_CUDA(c, c->d_sl_ord.ensure((size_t)npts * sizeof(unsigned short)));
+        CGS_CUDA(c, c->d_sl_head.ensure((size_t)ntl * sl.head_words * sizeof(unsigned)));
+        CGS_CUDA(c, c->d_sl_mask.ensure((size_t)ntl * sl.R2 * tbx * sizeof(unsigned)));
+        sl.ord = c->d_sl_ord.as<unsigned short>();
+        sl.len = c->d_csr_cnt.as<unsigned>();   // the fill cursors are not needed any more
+        sl.off = c->d_sl_off.as<unsigned>();
+        sl.head = c->d_sl_head.as<unsigned>();
+        sl.lmask = c->d_sl_mask.as<unsigned>();
+        unsigned runs = 0;
+        CGS_CUDA(c, slices_order(sl, c->d_sl_off.as<unsigned>(), c->d_csr_tmp.as<unsigned>(), tmp, &runs, c->stream));
+        CGS_CUDA(c, c->d_sl_ent.ensure(std::max<size_t>(runs, 1) * 32 * sizeof(int2)));
+        sl.sell = c->d_sl_ent.as<int2>();
+        CGS_CUDA(c, slices_fill(sl, c->stream));
+    }
     int bad = 0;
     CGS_CUDA(c, cudaMemcpyAsync(&bad, c->d_flag.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CGS_CUDA(c, cudaStreamSynchronize(c->stream));
     c->d_csr_cnt.release();   // the counts / fill cursors are not needed after the build
+    if (list == 2) c->d_csr_ent.release();   // the slices hold them
     if (bad) return CGS_OK;   // a tap outside the lists: keep the tiled kernel
     c->csr_pts = npts;
     c->csr_entries = ne;
@@ -563,6 +593,11 @@ bool fused_spread_applies(const cgs_ctx* c)
 // The forward grid holds quads of coils (fwd_x_quad.cuh) from three coils on;
 // with one or two, coil planes (a quad would be mostly padding).
 bool quad_grid(const cgs_ctx* c) { return c->nch >= 3; }
+// The spreading into the quad grid: where at most a third of it is padding
+// (not with five coils, whose second quad holds one: gather and x pass of a
+// 128 x 176 x 96 grid 0.22 ms against 0.20 by rows into coil planes)
+bool quad_spread(const cgs_ctx* c) { return quad_grid(c) && 12 * ((c->nch + 3) / 4) <= 4 * c->nch; }
+int spread_variant(const cgs_ctx* c) { return c->spread_wpp ? c->spread_wpp : quad_spread(c) ? 6 : 8; }
 // values of a bin's forward grid
 long long fwd_grid_elems(const cgs_ctx* c)
 {
@@ -584,7 +619,7 @@ int build_touch_mask(cgs_ctx* c)
     const int words = a.nsub * a.R1 * ((a.R2 + 3) / 4);
     CGS_CUDA(c, c->d_touch.ensure((size_t)a.ntl * words * sizeof(unsigned)));
     a.col_tile = c->d_col_tile.as<int>();
-    a.tb = c->csr_list == 1 ? c->sup_tb : c->spr_tb;
+    a.tb = c->csr_list >= 1 ? c->sup_tb : c->spr_tb;
     a.Gx = c->G[0];
     a.ncol = (long long)c->G[1] * c->G[2];
     a.ptr = c->d_csr_ptr.as<unsigned>();
@@ -599,7 +634,9 @@ int build_touch_mask(cgs_ctx* c)
 int ensure_csr(cgs_ctx* c)
 {
     if (!c->sup_built) return CGS_OK;
-    const int want = (c->spread_wpp == 8 && fused_spread_applies(c)) ? 1 : 0;
+    const int v = spread_variant(c);
+    if (v < 6 && c->csr_valid) return CGS_OK;   // not read by these
+    const int want = v == 8 && fused_spread_applies(c) ? 1 : v != 7 && quad_spread(c) ? 2 : 0;
     if (c->csr_list == want && c->csr_valid) return CGS_OK;
     drop_graphs(c);
     return build_csr(c, want);
@@ -737,6 +774,7 @@ int rebuild_bins(cgs_ctx* c)
     c->setup_ms[2] = ms_since(t0);
     t0 = clk::now();
     c->csr_list = -1;
+    c->csr_valid = false;
     c->touch_words = 0;
     CGS_TRY(ensure_csr(c));
     CGS_TRY(build_touch_mask(c));
@@ -988,8 +1026,49 @@ int adj_chain(cgs_ctx* c, int b0, int nb, float2* q, long long q_bs, bool use_sm
         // variant 8: the gather fused with the adjoint x pass (the listed
         // tiles of 8 columns of a half-pruned x pass); where it does not
         // apply, the staged gather and the x pass run as variant 6
-        bool fused = false;
-        if (sup && c->spread_wpp == 8 && c->csr_valid && c->csr_list == 1 && fused_spread_applies(c)) {
+        bool fused = false, quads = false;
+        const int variant = spread_variant(c);
+        if (sup && variant >= 6 && c->csr_valid && c->csr_list == 2) {
+            // variant 6: the gather over the sliced matrix into the quad grid, and
+            // the adjoint x pass from it
+            SliceSpreadArgs qa{};
+            qa.head = c->d_sl_head.as<unsigned>();
+            qa.ord = c->d_sl_ord.as<unsigned short>();
+            qa.sell = c->d_sl_ent.as<int2>();
+            qa.tb = c->sup_tb;
+            qa.pts = Gx * c->sup_tb;
+            qa.head_words = slice_head_words(qa.pts);
+            qa.tiles = c->d_sup_tiles.as<int2>();
+            qa.j0 = c->h_sup_off[b0];
+            qa.nj = c->h_sup_off[b0 + nb] - c->h_sup_off[b0];
+            qa.bin0 = b0;
+            qa.B = (long long)Gy * Gz;
+            qa.Ng = c->Ng;
+            qa.yv = c->d_yv.as<float2>();
+            qa.nch = c->nch;
+            qa.out = c->d_grid.as<float2>();
+            CGS_LAUNCH(c, launch_spread_quad(qa, c->kahan, c->stream));
+            CGS_TRY(prepare_adj_slots(c, b0, nb, sup));
+            AdjXQuadArgs xa{};
+            xa.in = qa.out;
+            xa.Ng = c->Ng;
+            xa.lmask = c->d_sl_mask.as<unsigned>();
+            xa.tiles = qa.tiles + qa.j0;
+            xa.j0 = qa.j0;
+            xa.ntl = qa.nj;
+            xa.tb = qa.tb;
+            xa.bin0 = b0;
+            xa.nch = c->nch;
+            xa.B = qa.B;
+            xa.Lout = Ix;
+            xa.out_off = c->lo[0];
+            xa.out = c->d_ybuf_adj.as<float2>();
+            xa.out_bs = yb;
+            xa.tw = c->tw[0].as<float2>();
+            CGS_LAUNCH(c, launch_adj_x_quad(Gx, xa, c->stream));
+            quads = true;
+        }
+        if (sup && variant == 8 && c->csr_valid && c->csr_list == 1 && fused_spread_applies(c)) {
             CGS_TRY(prepare_adj_slots(c, b0, nb, sup));
             SpreadAdjxArgs fa{};
             fa.ptr = c->d_csr_ptr.as<unsigned>();
@@ -1018,9 +1097,9 @@ int adj_chain(cgs_ctx* c, int b0, int nb, float2* q, long long q_bs, bool use_sm
             }
         }
         c->spread_fused = fused;
-        if (fused) {
-            // the adjoint y pass reads what the fused kernel stored
-        } else if (sup && c->spread_wpp >= 6 && c->csr_valid) {
+        if (fused || quads) {
+            // the adjoint y pass reads what these stored
+        } else if (sup && variant >= 6 && c->csr_valid && c->csr_list != 2) {
             // gather over the transposed tap matrix: stores the listed tiles' points
             CsrSpreadArgs ca{};
             ca.grid = c->d_grid.as<float2>();
@@ -1044,15 +1123,15 @@ int adj_chain(cgs_ctx* c, int b0, int nb, float2* q, long long q_bs, bool use_sm
             if (ca.cc != 2 && ca.cc != 4 && ca.cc != 6 && ca.cc != 8) ca.cc = 0;
             ca.err = c->d_err.as<int>();
             // variants 6 (and 8): the matrix staged in shared memory; 7: read from global memory
-            CGS_LAUNCH(c, launch_spread_csr(ca, c->kahan, c->spread_wpp != 7, c->stream));
+            CGS_LAUNCH(c, launch_spread_csr(ca, c->kahan, variant != 7, c->stream));
         } else {
             // variants 6 / 7 without their matrix: the two-warps-per-plane tiled kernel
-            const int wpp = c->spread_wpp >= 6 ? 2 : c->spread_wpp;
+            const int wpp = variant >= 6 ? 2 : variant;
             if (wpp == 2 && sa.cc < 2) sa.cc = std::min(2, c->nch);
             CGS_LAUNCH(c, launch_spread(sa, c->ntiles, nb, c->kahan, wpp, c->stream));
         }
 
-        if (!fused) {
+        if (!fused && !quads) {
             CGS_TRY(prepare_adj_slots(c, b0, nb, sup));
             StridedPassArgs ax{};
             ax.in = c->d_grid.as<float2>();
@@ -2809,7 +2888,7 @@ int cgs_pipe_menon_dcf(cgs_ctx* c, int32_t iters, float* dcf, int32_t on_device)
     for (int it = 0; csr && it < iters; ++it)
         for (int g = 0; g < c->nbins; g += per) {
             const int nb = std::min(per, c->nbins - g);
-            const bool xl = c->csr_list == 1;
+            const bool xl = c->csr_list >= 1;
             const std::vector<long long>& off = xl ? c->h_sup_off : c->h_spr_off;
             PmArgs pa{};
             pa.ptr = c->d_csr_ptr.as<unsigned>();
@@ -2829,6 +2908,26 @@ int cgs_pipe_menon_dcf(cgs_ctx* c, int32_t iters, float* dcf, int32_t on_device)
             pa.w = w.as<float>();
             long long mx = 0;
             for (int b = g; b < g + nb; ++b) mx = std::max(mx, c->h_bin_off[b + 1] - c->h_bin_off[b]);
+            if (c->csr_list == 2) {
+                SliceSpreadArgs qa{};
+                qa.head = c->d_sl_head.as<unsigned>();
+                qa.ord = c->d_sl_ord.as<unsigned short>();
+                qa.sell = c->d_sl_ent.as<int2>();
+                qa.tb = c->sup_tb;
+                qa.pts = c->G[0] * c->sup_tb;
+                qa.head_words = slice_head_words(qa.pts);
+                qa.tiles = pa.tiles;
+                qa.j0 = pa.j0;
+                qa.nj = pa.nj;
+                qa.bin0 = g;
+                qa.B = (long long)c->G[1] * c->G[2];
+                qa.Ng = c->Ng;
+                qa.w = pa.w;
+                qa.rout = pa.grid;
+                CGS_LAUNCH(c, launch_pm_slices(qa, c->stream));
+                CGS_LAUNCH(c, launch_pm_interp(pa, mx, c->stream));
+                continue;
+            }
             CGS_LAUNCH(c, launch_pm_step(pa, mx, c->stream));
             ++c->launches;   // spreading, interpolation with the update
         }

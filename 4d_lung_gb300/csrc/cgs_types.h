@@ -259,6 +259,60 @@ struct CsrSpreadArgs {
     int* err;                  // error flag (a bounded wait of the staged form ran out)
 };
 
+// The transposed tap matrix of the listed x-pass tiles in slices: a tile's
+// points in falling order of their tap counts, 32 a slice; tap j of the
+// slice's point l at sell[(off + j) * 32 + l], padded with zero weights to the
+// longest of the 32.
+struct SliceArgs {
+    const unsigned* ptr;       // row offsets of the matrix, points p = J * pts + i
+    const int2* ent;
+    long long ntl;             // tiles
+    int tb, pts;               // columns per tile, points per tile (Gx * tb)
+    int head_words;            // per tile: offset of every slice and the end
+    int R1, R2;                // split of the x line
+    unsigned short* ord;       // [ntl * pts] the points in order
+    unsigned* len;             // [ntl * pts / 32 + 1] taps of each slice's longest point
+    const unsigned* off;       // exclusive sum of len (in runs of 32)
+    unsigned* head;            // [ntl * head_words]
+    unsigned* lmask;           // [ntl][R2][tb]: bit n1 of row group n2 and column: point (R2 n1 + n2, column) has taps
+    int2* sell;
+};
+
+// Gather over the sliced matrix into the quad grid (k_spread_quad), or of real
+// density weights into a real grid (k_pm_slices)
+struct SliceSpreadArgs {
+    const unsigned* head;
+    const unsigned short* ord;
+    const int2* sell;
+    int head_words, pts, tb;
+    const int2* tiles;         // listed x-pass tiles {bin, first column}, global index
+    long long j0, nj;          // the tiles of this launch
+    int bin0;                  // bin of grid slot 0
+    long long B, Ng;           // Gy * Gz, grid points
+    const float2* yv;          // [total samples][nch]
+    int nch;
+    float2* out;               // quad grid (FwdXQuadArgs)
+    const float* w;            // density weights [total samples]
+    float* rout;               // real grid [slot][Ng]
+};
+
+// Adjoint x pass from the quad grid (adj_x_quad.cuh) over the listed tiles
+// [j0, j0 + ntl): coil c of slot s, kept row l - out_off of column b at
+// out + (s * nch + c) * out_bs + (l - out_off) * B + b.
+struct AdjXQuadArgs {
+    const float2* in;          // quad grid
+    long long Ng;
+    const unsigned* lmask;     // SliceArgs, all tiles
+    const int2* tiles;         // of this launch
+    long long j0, ntl;
+    int tb, bin0, nch;
+    long long B;
+    int Lout, out_off;
+    float2* out;
+    long long out_bs;
+    const float2* tw;
+};
+
 // Spreading fused with the adjoint x pass (spread_adjx.cuh): the gather of
 // CsrSpreadArgs over listed tiles of 8 columns and Gx = L rows (grid and
 // coil_stride unused), then the output-pruned x transform into the adjoint

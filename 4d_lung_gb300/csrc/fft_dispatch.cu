@@ -15,7 +15,8 @@ namespace cgs {
     cudaError_t fft_toep_x_##L_(const StridedPassArgs& a, const float* P, long long p_bs, int nsub, int batch, \
                                 cudaStream_t s);                                                       \
     cudaError_t fft_spread_adjx_##L_(const SpreadAdjxArgs& a, bool kahan, cudaStream_t s);             \
-    cudaError_t fft_fwd_x_quad_##L_(const FwdXQuadArgs& a, cudaStream_t s);
+    cudaError_t fft_fwd_x_quad_##L_(const FwdXQuadArgs& a, cudaStream_t s);                            \
+    cudaError_t fft_adj_x_quad_##L_(const AdjXQuadArgs& a, cudaStream_t s);
 CGS_FFT_SIZES(CGS_DECLARE)
 
 static const int kSizes[] = {
@@ -249,6 +250,16 @@ cudaError_t launch_fwd_x_quad(int L, const FwdXQuadArgs& a, cudaStream_t s)
 {
     switch (L) {
 #define CGS_CASE(L_, R1_, R2_, G_) case L_: return fft_fwd_x_quad_##L_(a, s);
+        CGS_FFT_SIZES(CGS_CASE)
+#undef CGS_CASE
+    }
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_adj_x_quad(int L, const AdjXQuadArgs& a, cudaStream_t s)
+{
+    switch (L) {
+#define CGS_CASE(L_, R1_, R2_, G_) case L_: return fft_adj_x_quad_##L_(a, s);
         CGS_FFT_SIZES(CGS_CASE)
 #undef CGS_CASE
     }

@@ -4,7 +4,7 @@
 #include "launch.h"
 #include "fft_passes.cuh"
 #include "spread_adjx.cuh"
-#include "fwd_x_quad.cuh"
+#include "adj_x_quad.cuh"
 
 #ifndef CGS_FFT_GROUP
 #define CGS_FFT_GROUP 0
@@ -62,6 +62,7 @@ struct SizeImpl {
     static constexpr int NSTAGE_NI = 3;
     // forward x pass over quads of coils: unit widths of the two forms
     static constexpr int TBQ_IN = fft_quad_tile_cols(R1, R2, true), TBQ_NO = fft_quad_tile_cols(R1, R2, false);
+    static constexpr int TBQ_ADJ = 4;   // of the adjoint x pass from it
 
     template <int SIGN, int MODE, int TBK = TB, int NS = NSTAGE>
     static cudaError_t tma_attr(int smem)
@@ -89,6 +90,15 @@ struct SizeImpl {
             e = cudaFuncSetAttribute(k_fwd_x_quad<R1, R2, TBQ_NO, PRUNE_NONE>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)QuadLayout<R1, R2, TBQ_NO>::smem_bytes(L + 3));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_adj_x_quad<R1, R2, TBQ_ADJ, PRUNE_NONE>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)AdjQuadLayout<R1, R2, TBQ_ADJ>::smem_bytes);
+        if constexpr (HAS_OUT)
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k_adj_x_quad<R1, R2, TBQ_ADJ, PRUNE_OUT>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)AdjQuadLayout<R1, R2, TBQ_ADJ>::smem_bytes);
         if constexpr (HAS_IN)
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(k_fwd_x_quad<R1, R2, TBQ_IN, PRUNE_IN>,
@@ -211,6 +221,31 @@ struct SizeImpl {
         if constexpr (HAS_IN)
             if (4 * a.in_off == L && 2 * a.Lin == L) return quad_run<TBQ_IN, PRUNE_IN>(a, s);
         return quad_run<TBQ_NO, PRUNE_NONE>(a, s);
+    }
+    // adjoint x pass from the quad grid
+    template <int TBQ, int MODE>
+    static cudaError_t adj_quad_run(const AdjXQuadArgs& a, cudaStream_t s)
+    {
+        using Lay = AdjQuadLayout<R1, R2, TBQ>;
+        int per_sm = 0;
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adj_x_quad<R1, R2, TBQ, MODE>, Lay::NT,
+                                                                      Lay::smem_bytes);
+        if (e != cudaSuccess) return e;
+        const int nsub = a.tb / TBQ;
+        const long long per_quad = a.ntl * nsub, nunits = per_quad * ((a.nch + 3) / 4);
+        if (nunits <= 0) return cudaSuccess;
+        if (nunits >= 0x7fffffffLL) return cudaErrorInvalidValue;
+        const long long nblk = std::min<long long>(nunits, (long long)sm_count() * std::max(per_sm, 1));
+        k_adj_x_quad<R1, R2, TBQ, MODE><<<(unsigned)nblk, Lay::NT, Lay::smem_bytes, s>>>(a, (int)nunits, (int)per_quad,
+                                                                                        nsub);
+        return cudaGetLastError();
+    }
+    static cudaError_t adj_x_quad(const AdjXQuadArgs& a, cudaStream_t s)
+    {
+        if (a.nch < 1 || a.tb % TBQ_ADJ != 0) return cudaErrorInvalidValue;
+        if constexpr (HAS_OUT)
+            if (4 * a.out_off == L && 2 * a.Lout == L) return adj_quad_run<TBQ_ADJ, PRUNE_OUT>(a, s);
+        return adj_quad_run<TBQ_ADJ, PRUNE_NONE>(a, s);
     }
     // Toeplitz x stage (in place, rows L/4 .. 3L/4 in and out)
     static cudaError_t toep_x(StridedPassArgs a, const float* P, long long p_bs, int nsub, int batch, cudaStream_t s)
@@ -337,6 +372,7 @@ struct SizeImpl {
                                 cudaStream_t s);                                                       \
     cudaError_t fft_spread_adjx_##L_(const SpreadAdjxArgs& a, bool kahan, cudaStream_t s);             \
     cudaError_t fft_fwd_x_quad_##L_(const FwdXQuadArgs& a, cudaStream_t s);                            \
+    cudaError_t fft_adj_x_quad_##L_(const AdjXQuadArgs& a, cudaStream_t s);                            \
     CGS_DEFINE_IF_##G_(L_, R1_, R2_)
 
 #define CGS_BODY(L_, R1_, R2_)                                                                      \
@@ -356,7 +392,9 @@ struct SizeImpl {
     cudaError_t fft_spread_adjx_##L_(const SpreadAdjxArgs& a, bool kahan, cudaStream_t s)              \
     { return SizeImpl<R1_, R2_>::spread_adjx(a, kahan, s); }                                         \
     cudaError_t fft_fwd_x_quad_##L_(const FwdXQuadArgs& a, cudaStream_t s)                             \
-    { return SizeImpl<R1_, R2_>::fwd_x_quad(a, s); }
+    { return SizeImpl<R1_, R2_>::fwd_x_quad(a, s); }                                                 \
+    cudaError_t fft_adj_x_quad_##L_(const AdjXQuadArgs& a, cudaStream_t s)                             \
+    { return SizeImpl<R1_, R2_>::adj_x_quad(a, s); }
 
 #if CGS_FFT_GROUP == 0
 #define CGS_DEFINE_IF_0(L, R1, R2) CGS_BODY(L, R1, R2)

@@ -31,3 +31,7 @@ constexpr int fft_quad_tile_cols(int r1, int r2, bool half_in)
 // spreading fused with the adjoint x pass (spread_adjx.cuh): threads per
 // block, columns per tile (the x passes' narrow tiles)
 constexpr int SAX_NT = 1024, SAX_TB = 8;
+
+// words of a tile's slice offsets (one slice per 32 of its points and the end),
+// rounded up to 16 bytes
+constexpr int slice_head_words(int pts) { return (pts / 32 + 1 + 3) & ~3; }

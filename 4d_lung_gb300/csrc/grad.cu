@@ -662,6 +662,11 @@ cudaError_t launch_pm_step(const PmArgs& a, long long max_bin, cudaStream_t s)
 {
     const long long np = a.nj * a.G[0] * a.tb;
     if (np > 0) k_pm_spread<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(a);
+    return launch_pm_interp(a, max_bin, s);
+}
+
+cudaError_t launch_pm_interp(const PmArgs& a, long long max_bin, cudaStream_t s)
+{
     if (max_bin > 0) k_pm_interp<<<dim3((unsigned)((max_bin + 127) / 128), (unsigned)a.nbins), 128, 0, s>>>(a);
     return cudaGetLastError();
 }

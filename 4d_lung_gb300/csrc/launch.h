@@ -39,6 +39,7 @@ int fft_quad_cols(int L, int lo, int I, int* R1, int* R2);
 
 // One launch per pass; `batch` items along blockIdx.y.
 cudaError_t launch_strided(int L, int sign, const StridedPassArgs& a, int A, int batch, cudaStream_t s);
+cudaError_t launch_adj_x_quad(int L, const AdjXQuadArgs& a, cudaStream_t s);
 cudaError_t launch_fwd_x_quad(int L, const FwdXQuadArgs& a, cudaStream_t s);
 cudaError_t launch_contig(int L, int sign, const ContigPassArgs& a, int batch, cudaStream_t s);
 cudaError_t launch_fwd_z(int L, const FwdZArgs& a, int batch, cudaStream_t s);
@@ -66,6 +67,13 @@ cudaError_t csr_count_and_scan(const CsrBuildArgs& a, long long npts, unsigned* 
                                size_t scan_tmp_elems, unsigned long long* entries, cudaStream_t s);
 cudaError_t csr_fill_and_order(const CsrBuildArgs& a, long long npts, cudaStream_t s);
 size_t csr_scan_tmp_elems(long long n);
+// The matrix in slices (SliceArgs): order, lengths and line masks, then (after
+// the lengths' sum *runs, in runs of 32 entries) headers and entries.
+cudaError_t slices_order(const SliceArgs& a, unsigned* off, unsigned* scan_tmp, size_t scan_tmp_elems,
+                         unsigned* runs, cudaStream_t s);
+cudaError_t slices_fill(const SliceArgs& a, cudaStream_t s);
+cudaError_t launch_spread_quad(const SliceSpreadArgs& a, bool kahan, cudaStream_t s);
+cudaError_t launch_pm_slices(const SliceSpreadArgs& a, cudaStream_t s);
 cudaError_t launch_touch_mask(const TouchMaskArgs& a, cudaStream_t s);
 cudaError_t launch_spread_csr(const CsrSpreadArgs& a, bool kahan, bool staged, cudaStream_t s);
 
@@ -137,6 +145,8 @@ cudaError_t launch_check_finite(const double* v, long long n, int* bad, cudaStre
 cudaError_t launch_pair_grad(const PairGradArgs& a, cudaStream_t s);
 // one iteration w <- w / (C w) of the bins of a; max_bin: their longest bin
 cudaError_t launch_pm_step(const PmArgs& a, long long max_bin, cudaStream_t s);
+// its second half alone (after launch_pm_slices)
+cudaError_t launch_pm_interp(const PmArgs& a, long long max_bin, cudaStream_t s);
 // out[ns] (zeroed here) = the weights over each bin's maximum, by global index;
 // a sample in several bins gets the last one's.  mx [nbins], owner [ns]: scratch
 cudaError_t launch_pm_finish(const float* w, const int* sorted, const long long* bin_off, int nbins, long long max_bin,

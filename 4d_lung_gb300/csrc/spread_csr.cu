@@ -127,6 +127,110 @@ cudaError_t launch_touch_mask(const TouchMaskArgs& a, cudaStream_t s)
 }
 
 // ---------------------------------------------------------------------------
+// slices (SliceArgs)
+// ---------------------------------------------------------------------------
+
+// One block per tile: thread t holds the points [t per, (t + 1) per), a stable
+// counting sort over ORD_CLASSES classes of tap counts (0, 1-2, 3-4, ...,
+// the last open).  The class counters are 16-bit fields of three 64-bit words.
+constexpr int ORD_T = 256, ORD_CLASSES = 12;
+
+__global__ void __launch_bounds__(ORD_T) k_point_order(const unsigned* __restrict__ ptr, int pts,
+                                                       unsigned short* __restrict__ ord)
+{
+    __shared__ unsigned long long s_w[ORD_T / 32][3];
+    const unsigned* p = ptr + (long long)blockIdx.x * pts;
+    const int per = (pts + ORD_T - 1) / ORD_T;
+    const int i0 = min((int)threadIdx.x * per, pts), i1 = min(i0 + per, pts);
+    auto cls = [&](int i) { return ORD_CLASSES - 1 - (int)min((p[i + 1] - p[i] + 1) / 2, (unsigned)ORD_CLASSES - 1); };
+    unsigned long long n[3] = {0, 0, 0};
+    for (int i = i0; i < i1; ++i) {
+        const int k = cls(i);
+#pragma unroll
+        for (int w = 0; w < 3; ++w) n[w] += k / 4 == w ? 1ull << (16 * (k % 4)) : 0ull;
+    }
+    // inclusive scan over the block (fields stay below 2^16: pts <= 16384)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long inc[3];
+#pragma unroll
+    for (int w = 0; w < 3; ++w) {
+        inc[w] = n[w];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long o = __shfl_up_sync(0xffffffffu, inc[w], d);
+            if (lane >= d) inc[w] += o;
+        }
+        if (lane == 31) s_w[warp][w] = inc[w];
+    }
+    __syncthreads();
+    unsigned long long tot[3] = {0, 0, 0};
+    for (int v = 0; v < ORD_T / 32; ++v)
+#pragma unroll
+        for (int w = 0; w < 3; ++w) {
+            if (v < warp) inc[w] += s_w[v][w];
+            tot[w] += s_w[v][w];
+        }
+    int pos[ORD_CLASSES], base = 0;
+#pragma unroll
+    for (int k = 0; k < ORD_CLASSES; ++k) {
+        pos[k] = base + (int)(((inc[k / 4] - n[k / 4]) >> (16 * (k % 4))) & 0xffff);
+        base += (int)((tot[k / 4] >> (16 * (k % 4))) & 0xffff);
+    }
+    unsigned short* o = ord + (long long)blockIdx.x * pts;
+    for (int i = i0; i < i1; ++i) {
+        const int k = cls(i);
+#pragma unroll
+        for (int q = 0; q < ORD_CLASSES; ++q)
+            if (k == q) o[pos[q]++] = (unsigned short)i;
+    }
+}
+
+// one warp per slice: the taps of its longest point
+__global__ void __launch_bounds__(256) k_slice_len(SliceArgs a)
+{
+    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31, per = a.pts / 32;
+    if (w >= a.ntl * per) return;
+    const unsigned* p = a.ptr + (w / per) * a.pts + a.ord[w * 32 + lane];
+    const unsigned n = __reduce_max_sync(0xffffffffu, p[1] - p[0]);
+    if (lane == 0) a.len[w] = n;
+}
+
+// one warp per slice: its entries and its word of the tile's header
+__global__ void __launch_bounds__(256) k_slice_fill(SliceArgs a)
+{
+    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31, per = a.pts / 32;
+    if (w >= a.ntl * per) return;
+    const long long J = w / per;
+    const int sl = (int)(w - J * per);
+    const unsigned o0 = a.off[w], o1 = a.off[w + 1];
+    unsigned* h = a.head + J * a.head_words;
+    if (lane == 0) h[sl] = o0;
+    if (sl == per - 1)
+        for (int q = per + lane; q < a.head_words; q += 32) h[q] = o1;
+    const unsigned* p = a.ptr + J * a.pts + a.ord[w * 32 + lane];
+    const unsigned e0 = p[0], n = p[1] - e0;
+    for (unsigned j = 0; j < o1 - o0; ++j)
+        a.sell[(long long)(o0 + j) * 32 + lane] = j < n ? a.ent[e0 + j] : make_int2(0, 0);
+}
+
+// one thread per (tile, n2, column)
+__global__ void __launch_bounds__(256) k_line_mask(SliceArgs a)
+{
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= a.ntl * a.R2 * a.tb) return;
+    const int col = (int)(e % a.tb), n2 = (int)((e / a.tb) % a.R2);
+    const unsigned* p = a.ptr + (e / (a.R2 * a.tb)) * a.pts;
+    unsigned m = 0;
+    for (int n1 = 0; n1 < a.R1; ++n1) {
+        const int i = (a.R2 * n1 + n2) * a.tb + col;
+        if (p[i + 1] > p[i]) m |= 1u << n1;
+    }
+    a.lmask[e] = m;
+}
+
+// ---------------------------------------------------------------------------
 // exclusive scan of unsigned counts (three-level block scan)
 // ---------------------------------------------------------------------------
 constexpr int SCAN_T = 512, SCAN_PER = 4, SCAN_CHUNK = SCAN_T * SCAN_PER;
@@ -197,6 +301,33 @@ static cudaError_t scan_exclusive(const unsigned* in, long long n, unsigned* out
     e = scan_exclusive(sums, nchunk, sums_scan, tmp + 2 * nchunk, s);
     if (e != cudaSuccess) return e;
     k_scan_add<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(out, n, sums_scan);
+    return cudaGetLastError();
+}
+
+cudaError_t slices_order(const SliceArgs& a, unsigned* off, unsigned* scan_tmp, size_t scan_tmp_elems,
+                         unsigned* runs, cudaStream_t s)
+{
+    *runs = 0;
+    const long long nsl = a.ntl * (a.pts / 32);
+    if (a.pts > 16384 || a.pts % 32 != 0 || a.R1 > 32 || a.ntl > 0x7fffffffLL ||
+        scan_tmp_elems < csr_scan_tmp_elems(nsl + 1))
+        return cudaErrorInvalidValue;
+    if (nsl == 0) return cudaSuccess;
+    k_point_order<<<(unsigned)a.ntl, ORD_T, 0, s>>>(a.ptr, a.pts, a.ord);
+    k_slice_len<<<(unsigned)((nsl + 7) / 8), 256, 0, s>>>(a);
+    k_line_mask<<<(unsigned)((a.ntl * a.R2 * a.tb + 255) / 256), 256, 0, s>>>(a);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemsetAsync(a.len + nsl, 0, sizeof(unsigned), s);
+    if (e == cudaSuccess) e = scan_exclusive(a.len, nsl + 1, off, scan_tmp, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(runs, off + nsl, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
+cudaError_t slices_fill(const SliceArgs& a, cudaStream_t s)
+{
+    const long long nsl = a.ntl * (a.pts / 32);
+    if (nsl == 0) return cudaSuccess;
+    k_slice_fill<<<(unsigned)((nsl + 7) / 8), 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -545,6 +676,171 @@ static cudaError_t spread_csr_staged_run(const CsrSpreadArgs& a, cudaStream_t s)
     if (nunits >= 0x7fffffffLL) return cudaErrorInvalidValue;
     const long long nblk = std::min<long long>(nunits, (long long)sm_count_csr() * std::max(per_sm, 1));
     k_spread_csr_staged<CC, KAHAN><<<(unsigned)nblk, nt, smem, s>>>(a, (int)nunits);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// The gather over the sliced matrix into the quad grid.  Block (tile, quad),
+// quads fastest; a warp takes slices warp, warp + 8, ... of the tile: lane l
+// owns the slice's point l and reads its taps as one 256-byte run per tap with
+// the other lanes, the sample's four coils as one 32-byte load (VM 4: coil
+// counts that are multiples of 4), two 16-byte (even) or four 8-byte loads.
+// Each point sums its taps in row order with k_spread_csr's operations (the
+// same bits) and is stored as one 32-byte sector; points without taps are not
+// stored (the adjoint x pass does not read them).  No shared memory and no
+// barriers, so that 48 warps per SM hide the loads.
+// ---------------------------------------------------------------------------
+template <int VM>
+CGS_D void load_quad(const float2* __restrict__ y, int nc, float (&v)[8])
+{
+    if constexpr (VM == 4) {
+        asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                     : "l"(y));
+    } else if constexpr (VM == 2) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(y));
+        float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (nc > 2) b = __ldg(reinterpret_cast<const float4*>(y) + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float2 t = c < nc ? __ldg(y + c) : make_float2(0.f, 0.f);
+            v[2 * c] = t.x;
+            v[2 * c + 1] = t.y;
+        }
+    }
+}
+
+// entries are read once per launch and quad: kept out of L1, which holds samples
+CGS_D int2 load_entry(const int2* p)
+{
+    int2 e;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(e.x), "=r"(e.y) : "l"(p));
+    return e;
+}
+
+constexpr int SQ_WARPS = 8;
+
+template <int VM, bool KAHAN>
+__global__ void __launch_bounds__(32 * SQ_WARPS, KAHAN ? 4 : 6) k_spread_quad(SliceSpreadArgs a)
+{
+    const int nq = (a.nch + 3) / 4;
+    const long long J = a.j0 + blockIdx.x / (unsigned)nq;
+    const int q = (int)(blockIdx.x % (unsigned)nq);
+    const int nc = min(4, a.nch - 4 * q);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned* head = a.head + J * a.head_words;
+    const int2 t = a.tiles[J];
+    const float2* yv = a.yv + 4 * q;
+    float2* out = a.out + ((long long)(t.x - a.bin0) * nq + q) * a.Ng * 4;
+    for (int sl = warp; sl < a.pts / 32; sl += SQ_WARPS) {
+        const unsigned o0 = __ldg(head + sl);
+        const int n = (int)(__ldg(head + sl + 1) - o0);
+        if (n == 0) break;   // slices come in falling order of length
+        const int2* ep = a.sell + (long long)o0 * 32 + lane;
+        const int pt = a.ord[J * a.pts + sl * 32 + lane];
+        float acc[8], cmp[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[c] = cmp[c] = 0.f;
+        auto add = [&](const float (&v)[8], float w) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                if (KAHAN) {
+                    // y = v w - e;  s = t + y;  e = (s - t) - y;  t = s
+                    const float y = fmaf(v[c], w, -cmp[c]), u = __fadd_rn(acc[c], y);
+                    cmp[c] = __fsub_rn(__fsub_rn(u, acc[c]), y);
+                    acc[c] = u;
+                } else {
+                    acc[c] = fmaf(v[c], w, acc[c]);
+                }
+            }
+        };
+        // two taps at a time, the next two entries ahead; a zero weight is padding
+        int2 e0 = load_entry(ep), e1 = n > 1 ? load_entry(ep + 32) : make_int2(0, 0);
+        const bool any = e0.y != 0;
+        for (int j = 0; j < n; j += 2) {
+            const int2 p = e0, r = e1;
+            ep += 64;
+            e0 = j + 2 < n ? load_entry(ep) : make_int2(0, 0);
+            e1 = j + 3 < n ? load_entry(ep + 32) : make_int2(0, 0);
+            float vp[8], vr[8];
+            if (p.y != 0) load_quad<VM>(yv + (long long)p.x * a.nch, nc, vp);
+            if (r.y != 0) load_quad<VM>(yv + (long long)r.x * a.nch, nc, vr);
+            if (p.y != 0) add(vp, __int_as_float(p.y));
+            if (r.y != 0) add(vr, __int_as_float(r.y));
+        }
+        if (!any) continue;
+        if (KAHAN) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) acc[c] = __fsub_rn(acc[c], cmp[c]);
+        }
+        const int x = pt / a.tb;
+        float4* o = reinterpret_cast<float4*>(out + ((long long)x * a.B + t.y + (pt - x * a.tb)) * 4);
+        o[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        o[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    }
+}
+
+cudaError_t launch_spread_quad(const SliceSpreadArgs& a, bool kahan, cudaStream_t s)
+{
+    const long long n = a.nj * ((a.nch + 3) / 4);
+    if (n == 0) return cudaSuccess;
+    if (n > 0x7fffffffLL || (reinterpret_cast<uintptr_t>(a.yv) & 31)) return cudaErrorInvalidValue;
+    const int vm = a.nch % 4 == 0 ? 4 : a.nch % 2 == 0 ? 2 : 1;
+    const unsigned nb = (unsigned)n;
+    const int nt = 32 * SQ_WARPS;
+    if (kahan) {
+        if (vm == 4) k_spread_quad<4, true><<<nb, nt, 0, s>>>(a);
+        else if (vm == 2) k_spread_quad<2, true><<<nb, nt, 0, s>>>(a);
+        else k_spread_quad<1, true><<<nb, nt, 0, s>>>(a);
+    } else {
+        if (vm == 4) k_spread_quad<4, false><<<nb, nt, 0, s>>>(a);
+        else if (vm == 2) k_spread_quad<2, false><<<nb, nt, 0, s>>>(a);
+        else k_spread_quad<1, false><<<nb, nt, 0, s>>>(a);
+    }
+    return cudaGetLastError();
+}
+
+// The real gather of the density weights: the same slices
+__global__ void __launch_bounds__(32 * SQ_WARPS) k_pm_slices(SliceSpreadArgs a)
+{
+    const long long J = a.j0 + blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned* head = a.head + J * a.head_words;
+    const int2 t = a.tiles[J];
+    for (int sl = warp; sl < a.pts / 32; sl += SQ_WARPS) {
+        const unsigned o0 = __ldg(head + sl);
+        const int n = (int)(__ldg(head + sl + 1) - o0);
+        if (n == 0) break;
+        const int2* ep = a.sell + (long long)o0 * 32 + lane;
+        const int pt = a.ord[J * a.pts + sl * 32 + lane];
+        float acc = 0.f;
+        bool any = false;
+        for (int j = 0; j < n; j += 4) {
+            int2 e[4];
+            float v[4];
+#pragma unroll
+            for (int l = 0; l < 4; ++l) e[l] = j + l < n ? load_entry(ep + 32 * (j + l)) : make_int2(0, 0);
+#pragma unroll
+            for (int l = 0; l < 4; ++l) v[l] = e[l].y != 0 ? __ldg(a.w + e[l].x) : 0.f;
+#pragma unroll
+            for (int l = 0; l < 4; ++l)
+                if (e[l].y != 0) {
+                    acc = fmaf(v[l], __int_as_float(e[l].y), acc);
+                    any = true;
+                }
+        }
+        const int x = pt / a.tb;
+        if (any) a.rout[(long long)(t.x - a.bin0) * a.Ng + (long long)x * a.B + t.y + (pt - x * a.tb)] = acc;
+    }
+}
+
+cudaError_t launch_pm_slices(const SliceSpreadArgs& a, cudaStream_t s)
+{
+    if (a.nj == 0) return cudaSuccess;
+    k_pm_slices<<<(unsigned)a.nj, 32 * SQ_WARPS, 0, s>>>(a);
     return cudaGetLastError();
 }
 

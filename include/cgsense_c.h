@@ -313,14 +313,16 @@ int cgs_set_deterministic(cgs_ctx* ctx, int32_t on);
  * plane of a tile; 3: shared-memory atomics, only with determinism off;
  * 4 / 5: persistent and software-pipelined with one / two warps per plane;
  * 6: a gather over the transposed tap matrix, built with the bins when
- * sample-support pruning is on -- without it variant 2 runs -- whose row
- * offsets and taps are staged in shared memory by bulk copies; 7: the same
- * gather reading the matrix from global memory; for 6 and 7 spread_cc is the
- * coils per thread, 2, 4, 6 or 8, 0 by the coil count; 8 (default): the
- * staged gather fused with the adjoint x pass, one block per listed
- * 8-column tile and chunk of spread_cc coils (2, 4 or 6, 0 by the coil
- * count), the grid kept in shared memory -- where the grid is not twice the
- * image along x, or the coil count has no such chunk, variant 6 runs),
+ * sample-support pruning is on -- without it variant 2 runs: from three coils
+ * on (not with five) over the matrix in slices into a grid of coil quads that
+ * the adjoint x pass reads, else over rows whose offsets and taps are staged
+ * in shared memory by bulk copies, spread_cc coils per thread (2, 4, 6 or 8,
+ * 0 by the coil count); 7: the gather over rows read from global memory, with
+ * the same spread_cc; 8: the staged gather fused with the adjoint x pass, one
+ * block per listed 8-column tile and chunk of spread_cc coils (2, 4 or 6, 0 by
+ * the coil count), the grid kept in shared memory -- where the grid is not
+ * twice the image along x, or the coil count has no such chunk, variant 6
+ * runs.  The default is 6 in its sliced form where that applies, else 8),
  * coils per interpolation thread (1, 2, 4, 6, 8; with coils in quads 6 and
  * 8 count as 4).  Variants 1, 2, 4, 5, 6,
  * 7, 8 and every interpolation shape give bitwise-identical results. */

@@ -44,3 +44,33 @@ def test_quads_equal_coil_planes_bitwise(gpu_lib, cgs, img, grid, nch, kb_w, pru
     for cc in (1, 2, 4):
         r.set_launch_shape(0, 8, cc)
         assert np.array_equal(r.nufft_fwd(x), y), cc
+
+
+@pytest.mark.parametrize("img,grid,nch,kb_w", CASES)
+@pytest.mark.parametrize("compensated", [False, True])
+def test_sliced_gather_equals_tiled_kernel_bitwise(gpu_lib, cgs, img, grid, nch, kb_w, compensated):
+    """The gather over the sliced matrix and the adjoint x pass from the quad
+    grid against the tiled spreading kernel and the pass from coil planes, with
+    a crowded spot (slices of very different lengths) and two bins."""
+    rng = np.random.default_rng(6)
+    k = np.concatenate([0.5 + 0.15 * rng.standard_normal((500, 3)).clip(-3, 3), rng.uniform(0, 1, (100, 3)),
+                        0.5 + 0.002 * rng.standard_normal((300, 3))])
+    k[:6] = [[0, 0, 0], [1, 1, 1], [0, 1, 0.5], [1, 0, 0.5], [0.5, 0, 1], [0.5, 1, 0]]
+    y = (rng.standard_normal((nch, len(k))) + 1j * rng.standard_normal((nch, len(k)))).astype(np.complex64)
+    maps = (rng.standard_normal((nch,) + img) + 1j * rng.standard_normal((nch,) + img)).astype(np.complex64)
+    r = cgs.Reco(img, grid, nch, kb_w=kb_w, kb_b=9.0)
+    r.set_trajectory(k)
+    r.set_smaps(maps)
+    r.set_precision(compensated)
+    got = r.nufft_adj(y)
+    r.set_launch_shape(0, 6, 2)
+    assert np.array_equal(got, r.nufft_adj(y))
+    r.set_launch_shape(0, 1, 2)
+    assert np.abs(got).max() > 0
+    assert np.array_equal(got, r.nufft_adj(y))
+    r.set_bins([np.arange(0, 450), np.arange(450, 900)])
+    r.set_launch_shape(0, 6, 2)
+    x6, res6, _ = r.cg_sense_batched(y, 0.0, 3)
+    r.set_launch_shape(0, 1, 2)
+    x1, res1, _ = r.cg_sense_batched(y, 0.0, 3)
+    assert np.array_equal(x6, x1) and np.array_equal(res6, res1)
