@@ -148,6 +148,8 @@ struct cgs_ctx {
                                              // over the x passes' (quad grid); -1 not built
     // transposed tap matrix of the listed tiles' points (spreading variant 6)
     bool csr_valid = false;
+    DevBuf d_col_mark;                       // per bin and grid column: some sample's support reaches it
+    bool tile_lists_built = false;           // ensure_tile_lists
     long long csr_pts = 0;
     unsigned long long csr_entries = 0;
     DevBuf d_col_tile, d_csr_cnt, d_csr_ptr, d_csr_ent, d_csr_tmp;
@@ -320,7 +322,8 @@ std::vector<double> deapod_axis(const cgs_params& p, int n)
 }
 
 // Host-side bin preparation.  Samples are sorted by their home spreading
-// tile (the tile of the nearest grid point).  Each tile then gets the list of
+// tile (the tile of the nearest grid point).  For the tiled spreading kernels
+// (ensure_tile_lists: only where one will run) each tile gets the list of
 // the samples whose 5-point support touches it, ordered by nearest x (stable
 // in sorted position), and per x plane of the tile the range of that list
 // whose support covers the plane.  The lists use the nearest points of the
@@ -332,7 +335,6 @@ struct BinPrep {
     std::vector<int> plane_rng;   // [ntiles][TILE_X][2]
     std::vector<int> sup_cols;        // first column of each x-pass tile the samples touch
     std::vector<int> spr_cols;        // the same for the spreading gather's wider tiles
-    std::vector<int> live;            // spreading tiles holding a supported column
 };
 
 void nearest_point(const double* kk, const int* G, int* nr)
@@ -434,55 +436,39 @@ void tile_lists(const cgs_ctx* c, const unsigned* nearest, long long n, BinPrep&
 // support reaches is never read after the forward x pass, and the adjoint x
 // pass transforms zeros there.  The x passes work on tiles of tb consecutive
 // columns of the flattened [Gy][Gz] plane: the tiles holding a supported
-// column are listed (sup_cols); the spreading stores the grid tiles whose
-// (y, z) extent meets a listed column (live).
-void support_lists(const cgs_ctx* c, const unsigned* nearest, long long n, int tb, int tbs, BinPrep& out)
+// column (col, marked on the device) are listed (sup_cols), and the spreading
+// gather's tiles of tbs columns (tb divides tbs; spr_cols).
+void support_lists(const unsigned char* col, long long ncol, int tb, int tbs, BinPrep& out)
+{
+    auto list = [&](int w, std::vector<int>& cols) {
+        cols.clear();
+        for (long long b0 = 0; b0 < ncol; b0 += w) {
+            const long long b1 = std::min(ncol, b0 + w);
+            bool any = false;
+            for (long long b = b0; b < b1 && !any; ++b) any = col[b] != 0;
+            if (any) cols.push_back((int)b0);
+        }
+    };
+    list(tb, out.sup_cols);
+    list(tbs, out.spr_cols);
+}
+
+// Spreading tiles whose (y, z) extent holds a listed column: the adjoint x
+// pass reads those columns at every x, so the tiled kernels store these tiles
+// (with zeros where no sample reaches); no other grid point is ever read.
+std::vector<int> live_tiles_of(const cgs_ctx* c, int bin)
 {
     const int Gy = c->G[1], Gz = c->G[2];
     const long long ncol = (long long)Gy * Gz;
-    std::vector<unsigned char> col(ncol, 0);
-    for (long long j = 0; j < n; ++j) {
-        const int ny = (int)((nearest[j] >> 11) & 2047u), nz = (int)(nearest[j] >> 22);
-        const int y0 = std::max(ny - 2, 0), y1 = std::min(ny + 2, Gy - 1);
-        const int z0 = std::max(nz - 2, 0), z1 = std::min(nz + 2, Gz - 1);
-        for (int y = y0; y <= y1; ++y)
-            for (int z = z0; z <= z1; ++z) col[(long long)y * Gz + z] = 1;
-    }
-    std::vector<unsigned char> listed(ncol, 0);   // column lies in a listed tile
-    out.sup_cols.clear();
-    for (long long b0 = 0; b0 < ncol; b0 += tb) {
-        const long long b1 = std::min(ncol, b0 + tb);
-        bool any = false;
-        for (long long b = b0; b < b1 && !any; ++b) any = col[b] != 0;
-        if (!any) continue;
-        out.sup_cols.push_back((int)b0);
-        for (long long b = b0; b < b1; ++b) listed[b] = 1;
-    }
-    // the spreading gather's tiles (tb divides tbs)
-    out.spr_cols.clear();
-    for (long long b0 = 0; b0 < ncol; b0 += tbs) {
-        const long long b1 = std::min(ncol, b0 + tbs);
-        bool any = false;
-        for (long long b = b0; b < b1 && !any; ++b) any = col[b] != 0;
-        if (any) out.spr_cols.push_back((int)b0);
-    }
-    // spreading tiles whose (y, z) extent holds a masked column: the adjoint
-    // x pass reads those columns at every x, so these tiles are stored (with
-    // zeros where no sample reaches); no other grid point is ever read
     std::vector<unsigned char> tcol((size_t)c->nty * c->ntz, 0);
-    for (int ty = 0; ty < c->nty; ++ty)
-        for (int tz = 0; tz < c->ntz; ++tz) {
-            bool any = false;
-            for (int y = ty * TILE_Y; y < std::min((ty + 1) * TILE_Y, Gy) && !any; ++y)
-                for (int z = tz * TILE_Z; z < std::min((tz + 1) * TILE_Z, Gz) && !any; ++z) {
-                    any = listed[(long long)y * Gz + z] != 0;
-                }
-            tcol[(size_t)ty * c->ntz + tz] = any;
-        }
-    out.live.clear();
+    for (long long J = c->h_sup_off[bin]; J < c->h_sup_off[bin + 1]; ++J)
+        for (long long f = c->h_sup_tiles[J].y; f < std::min(ncol, (long long)c->h_sup_tiles[J].y + c->sup_tb); ++f)
+            tcol[(size_t)(f / Gz / TILE_Y) * c->ntz + (f % Gz) / TILE_Z] = 1;
+    std::vector<int> live;
     for (int tx = 0; tx < c->ntx; ++tx)
         for (int j = 0; j < c->nty * c->ntz; ++j)
-            if (tcol[j]) out.live.push_back(tx * c->nty * c->ntz + j);
+            if (tcol[j]) live.push_back(tx * c->nty * c->ntz + j);
+    return live;
 }
 
 int upload(cgs_ctx* c, DevBuf& b, const void* h, size_t bytes)
@@ -685,10 +671,9 @@ int rebuild_bins(cgs_ctx* c)
     c->nbins = (int)c->bins.size();
     std::vector<BinPrep> prep(c->nbins);
     c->h_bin_off.assign(c->nbins + 1, 0);
-    for (int b = 0; b < c->nbins; ++b) {
-        sort_bin(c, c->bins[b], prep[b]);
-        c->h_bin_off[b + 1] = c->h_bin_off[b] + (long long)c->bins[b].size();
-    }
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int b = 0; b < c->nbins; ++b) sort_bin(c, c->bins[b], prep[b]);
+    for (int b = 0; b < c->nbins; ++b) c->h_bin_off[b + 1] = c->h_bin_off[b] + (long long)c->bins[b].size();
     c->total = c->h_bin_off[c->nbins];
     c->max_bin = 0;
     for (int b = 0; b < c->nbins; ++b) c->max_bin = std::max(c->max_bin, (long long)c->bins[b].size());
@@ -699,22 +684,13 @@ int rebuild_bins(cgs_ctx* c)
     CGS_TRY(upload(c, c->d_bin_off, c->h_bin_off.data(), c->h_bin_off.size() * sizeof(long long)));
     c->setup_ms[0] = ms_since(t0);
     t0 = clk::now();
-    // tap records (the device's nearest points decide the tile lists)
+    // tap records (the device's nearest points decide the lists)
     CGS_CUDA(c, c->d_rec.ensure(std::max<long long>(c->total, 1) * sizeof(TapRecord)));
     const KbParams kb = kb_params(c);
     CGS_CUDA(c, launch_tap_records(c->d_k.as<double>(), c->d_sorted.as<int>(), c->total, kb, c->d_rec.as<TapRecord>(),
                                    c->stream));
     c->drec_valid = false;
     c->tiles_stale = false;
-    std::vector<unsigned> nearest(std::max<long long>(c->total, 1));
-    {
-        DevBuf d_near;
-        CGS_CUDA(c, d_near.ensure(nearest.size() * sizeof(unsigned)));
-        CGS_CUDA(c, launch_record_nearest(c->d_rec.as<TapRecord>(), c->total, d_near.as<unsigned>(), c->stream));
-        CGS_CUDA(c, cudaMemcpyAsync(nearest.data(), d_near.p, nearest.size() * sizeof(unsigned), cudaMemcpyDeviceToHost,
-                                    c->stream));
-        CGS_CUDA(c, cudaStreamSynchronize(c->stream));
-    }
     c->setup_ms[1] = ms_since(t0);
     t0 = clk::now();
     // the x passes' tiles: 8 columns (64-byte rows) where both passes run
@@ -724,34 +700,33 @@ int rebuild_bins(cgs_ctx* c)
     if (tbx <= 0 || tbs % tbx != 0) tbs = tbx;
     c->sup_tb = tbx;
     c->spr_tb = tbs;
+    const long long ncol = (long long)c->G[1] * c->G[2];
+    if (tbx > 0) {
+        std::vector<unsigned char> col((size_t)c->nbins * ncol);
+        CGS_CUDA(c, c->d_col_mark.ensure(col.size()));
+        CGS_CUDA(c, launch_mark_columns(c->d_rec.as<TapRecord>(), c->total, c->d_bin_off.as<long long>(), c->nbins,
+                                        c->G, c->d_col_mark.as<unsigned char>(), c->stream));
+        CGS_CUDA(c, cudaMemcpyAsync(col.data(), c->d_col_mark.p, col.size(), cudaMemcpyDeviceToHost, c->stream));
+        CGS_CUDA(c, cudaStreamSynchronize(c->stream));
 #pragma omp parallel for schedule(dynamic, 1)
-    for (int b = 0; b < c->nbins; ++b) {
-        tile_lists(c, nearest.data() + c->h_bin_off[b], c->h_bin_off[b + 1] - c->h_bin_off[b], prep[b]);
-        if (tbx > 0)
-            support_lists(c, nearest.data() + c->h_bin_off[b], c->h_bin_off[b + 1] - c->h_bin_off[b], tbx, tbs,
-                          prep[b]);
+        for (int b = 0; b < c->nbins; ++b) support_lists(col.data() + (size_t)b * ncol, ncol, tbx, tbs, prep[b]);
     }
+    c->tile_lists_built = false;
     c->sup_built = false;
     c->h_sup_off.assign(c->nbins + 1, 0);
     c->h_spr_off.assign(c->nbins + 1, 0);
     if (tbx > 0) {
         std::vector<int2> tiles, spr;
-        std::vector<int> live;
-        c->h_live_off.assign(c->nbins + 1, 0);
         for (int b = 0; b < c->nbins; ++b) {
             for (int b0 : prep[b].sup_cols) tiles.push_back(make_int2(b, b0));
             c->h_sup_off[b + 1] = (long long)tiles.size();
             for (int b0 : prep[b].spr_cols) spr.push_back(make_int2(b, b0));
             c->h_spr_off[b + 1] = (long long)spr.size();
-            live.insert(live.end(), prep[b].live.begin(), prep[b].live.end());
-            c->h_live_off[b + 1] = (long long)live.size();
         }
         CGS_TRY(upload(c, c->d_sup_tiles, tiles.data(), std::max<size_t>(tiles.size(), 1) * sizeof(int2)));
         c->h_sup_tiles = tiles;
         CGS_TRY(upload(c, c->d_spr_tiles, spr.data(), std::max<size_t>(spr.size(), 1) * sizeof(int2)));
         c->h_spr_tiles = spr;
-        CGS_TRY(upload(c, c->d_live, live.data(), std::max<size_t>(live.size(), 1) * sizeof(int)));
-        CGS_TRY(upload(c, c->d_live_off, c->h_live_off.data(), c->h_live_off.size() * sizeof(long long)));
         c->sup_built = true;
         // row masks of the forward y pass: it stores row y of column z only
         // when the x pass lists the column tile starting at y * Gz + zs * tb,
@@ -780,22 +755,6 @@ int rebuild_bins(cgs_ctx* c)
     CGS_TRY(build_touch_mask(c));
     c->setup_ms[3] = ms_since(t0);
     t0 = clk::now();
-    std::vector<int> tile_ptr;
-    std::vector<int> tile_idx;
-    std::vector<int> plane_rng;
-    std::vector<long long> tp_off(c->nbins), ti_off(c->nbins);
-    for (int b = 0; b < c->nbins; ++b) {
-        tp_off[b] = (long long)tile_ptr.size();
-        tile_ptr.insert(tile_ptr.end(), prep[b].tile_ptr.begin(), prep[b].tile_ptr.end());
-        ti_off[b] = (long long)tile_idx.size();
-        tile_idx.insert(tile_idx.end(), prep[b].tile_idx.begin(), prep[b].tile_idx.end());
-        plane_rng.insert(plane_rng.end(), prep[b].plane_rng.begin(), prep[b].plane_rng.end());
-    }
-    CGS_TRY(upload(c, c->d_tile_ptr, tile_ptr.data(), tile_ptr.size() * sizeof(int)));
-    CGS_TRY(upload(c, c->d_tile_idx, tile_idx.data(), std::max<size_t>(tile_idx.size(), 1) * sizeof(int)));
-    CGS_TRY(upload(c, c->d_tile_ptr_off, tp_off.data(), tp_off.size() * sizeof(long long)));
-    CGS_TRY(upload(c, c->d_tile_idx_off, ti_off.data(), ti_off.size() * sizeof(long long)));
-    CGS_TRY(upload(c, c->d_plane_rng, plane_rng.data(), std::max<size_t>(plane_rng.size(), 2) * sizeof(int)));
     if (c->has_dcf) {
         std::vector<float> ds(c->total);
         for (long long j = 0; j < c->total; ++j) ds[j] = c->h_dcf[sorted[j]];
@@ -822,6 +781,59 @@ int rebuild_bins(cgs_ctx* c)
     return CGS_OK;
 }
 
+// Lists of the tiled spreading kernels (k_spread and its forms) from the
+// current tap records.  Built when one of them is going to run: the gathers
+// over the tap matrix do not read them, and building them took most of a
+// set-up (1 572 864 samples in one bin: 40 of 65 ms).
+int ensure_tile_lists(cgs_ctx* c)
+{
+    if (c->tile_lists_built) return CGS_OK;
+    std::vector<unsigned> nearest(std::max<long long>(c->total, 1));
+    DevBuf d_near;
+    CGS_CUDA(c, d_near.ensure(nearest.size() * sizeof(unsigned)));
+    CGS_CUDA(c, launch_record_nearest(c->d_rec.as<TapRecord>(), c->total, d_near.as<unsigned>(), c->stream));
+    CGS_CUDA(c, cudaMemcpyAsync(nearest.data(), d_near.p, nearest.size() * sizeof(unsigned), cudaMemcpyDeviceToHost,
+                                c->stream));
+    CGS_CUDA(c, cudaStreamSynchronize(c->stream));
+    std::vector<BinPrep> prep(c->nbins);
+    std::vector<std::vector<int>> live(c->nbins);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int b = 0; b < c->nbins; ++b) {
+        tile_lists(c, nearest.data() + c->h_bin_off[b], c->h_bin_off[b + 1] - c->h_bin_off[b], prep[b]);
+        if (c->sup_built) live[b] = live_tiles_of(c, b);
+    }
+    std::vector<int> tile_ptr;
+    std::vector<int> tile_idx;
+    std::vector<int> plane_rng;
+    std::vector<long long> tp_off(c->nbins), ti_off(c->nbins);
+    for (int b = 0; b < c->nbins; ++b) {
+        tp_off[b] = (long long)tile_ptr.size();
+        tile_ptr.insert(tile_ptr.end(), prep[b].tile_ptr.begin(), prep[b].tile_ptr.end());
+        ti_off[b] = (long long)tile_idx.size();
+        tile_idx.insert(tile_idx.end(), prep[b].tile_idx.begin(), prep[b].tile_idx.end());
+        plane_rng.insert(plane_rng.end(), prep[b].plane_rng.begin(), prep[b].plane_rng.end());
+    }
+    CGS_TRY(upload(c, c->d_tile_ptr, tile_ptr.data(), tile_ptr.size() * sizeof(int)));
+    CGS_TRY(upload(c, c->d_tile_idx, tile_idx.data(), std::max<size_t>(tile_idx.size(), 1) * sizeof(int)));
+    CGS_TRY(upload(c, c->d_tile_ptr_off, tp_off.data(), tp_off.size() * sizeof(long long)));
+    CGS_TRY(upload(c, c->d_tile_idx_off, ti_off.data(), ti_off.size() * sizeof(long long)));
+    CGS_TRY(upload(c, c->d_plane_rng, plane_rng.data(), std::max<size_t>(plane_rng.size(), 2) * sizeof(int)));
+    if (c->sup_built) {
+        std::vector<int> all;
+        c->h_live_off.assign(c->nbins + 1, 0);
+        for (int b = 0; b < c->nbins; ++b) {
+            all.insert(all.end(), live[b].begin(), live[b].end());
+            c->h_live_off[b + 1] = (long long)all.size();
+        }
+        CGS_TRY(upload(c, c->d_live, all.data(), std::max<size_t>(all.size(), 1) * sizeof(int)));
+        CGS_TRY(upload(c, c->d_live_off, c->h_live_off.data(), c->h_live_off.size() * sizeof(long long)));
+        CGS_CUDA(c, cudaStreamSynchronize(c->stream));   // the host vectors go out of scope
+    }
+    CGS_CUDA(c, cudaStreamSynchronize(c->stream));
+    c->tile_lists_built = true;
+    return CGS_OK;
+}
+
 // ---------------------------------------------------------------------------
 // chains
 // ---------------------------------------------------------------------------
@@ -829,6 +841,10 @@ int rebuild_bins(cgs_ctx* c)
 // The support lists describe the current tap records (not after
 // cgs_update_trajectory_d until the lists are rebuilt).
 bool support_pruned(const cgs_ctx* c) { return c->sup_prune && !c->tiles_stale && c->sup_built; }
+
+// Spreading now would run a tiled kernel (the choice of adj_chain, and of the
+// density weights, which need the matrix only)
+bool tiled_spread(const cgs_ctx* c) { return !(support_pruned(c) && spread_variant(c) >= 6 && c->csr_valid); }
 
 // Zero the adjoint y-buffer slots [0, nb) that held other bins' columns
 // before bins [b0, b0 + nb) are written there with pruning (the adjoint y
@@ -1017,7 +1033,7 @@ int adj_chain(cgs_ctx* c, int b0, int nb, float2* q, long long q_bs, bool use_sm
         sa.nty = c->nty;
         sa.ntz = c->ntz;
         sa.thresh = c->thresh;
-        if (sup) {
+        if (sup && c->tile_lists_built) {
             sa.live = c->d_live.as<int>();
             sa.live_off = c->d_live_off.as<long long>();
             for (int b = b0; b < b0 + nb; ++b)
@@ -1126,6 +1142,7 @@ int adj_chain(cgs_ctx* c, int b0, int nb, float2* q, long long q_bs, bool use_sm
             CGS_LAUNCH(c, launch_spread_csr(ca, c->kahan, variant != 7, c->stream));
         } else {
             // variants 6 / 7 without their matrix: the two-warps-per-plane tiled kernel
+            if (!c->tile_lists_built) return fail(c, CGS_ERR_STATE, "internal: tiled spreading without its lists");
             const int wpp = variant >= 6 ? 2 : variant;
             if (wpp == 2 && sa.cc < 2) sa.cc = std::min(2, c->nch);
             CGS_LAUNCH(c, launch_spread(sa, c->ntiles, nb, c->kahan, wpp, c->stream));
@@ -1570,6 +1587,7 @@ int check_ready(cgs_ctx* c, bool need_smaps, bool need_tiles = true)
     if (need_smaps && !c->smaps_set) return fail(c, CGS_ERR_STATE, "no coil maps set (cgs_set_smaps)");
     if (need_tiles && c->tiles_stale) c->bins_dirty = true;
     CGS_TRY(rebuild_bins(c));
+    if (need_tiles && tiled_spread(c)) CGS_TRY(ensure_tile_lists(c));
     if (c->toep_mode && (!c->toep_valid || c->toep_serial != c->traj_serial)) CGS_TRY(build_toeplitz(c));
     return CGS_OK;
 }
@@ -2589,6 +2607,7 @@ int cgs_autotune(cgs_ctx* c, float* times_ms, int32_t max_times, int32_t* n_time
                  int32_t* spread_wpp, int32_t* interp_cc)
 {
     CGS_TRY(check_ready(c, true));
+    CGS_TRY(ensure_tile_lists(c));   // the candidates hold the tiled kernels
     // the candidates are shapes of the gridded operator's kernels: timed with
     // the Toeplitz embedding off
     struct ModeGuard {
@@ -3056,6 +3075,7 @@ int cgs_support_stats(cgs_ctx* c, int64_t* listed_cols, int64_t* live_tiles)
     const bool sup = support_pruned(c);
     const long long ncol = (long long)c->G[1] * c->G[2];
     const int tbx = c->sup_tb;
+    if (live_tiles && sup) CGS_TRY(ensure_tile_lists(c));
     for (int b = 0; b < c->nbins; ++b) {
         if (listed_cols)
             listed_cols[b] = sup ? std::min(ncol, (c->h_sup_off[b + 1] - c->h_sup_off[b]) * (long long)tbx) : ncol;

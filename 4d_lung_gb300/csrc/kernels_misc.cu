@@ -104,6 +104,37 @@ cudaError_t launch_interp(const InterpArgs& a, long long max_bin_samples, int nb
     return cudaGetLastError();
 }
 
+// One thread per sample and y offset: five neighbouring columns (every store
+// writes the same value).
+__global__ void k_mark_columns(const TapRecord* __restrict__ rec, long long n, const long long* __restrict__ bin_off,
+                               int nbins, int Gy, int Gz, unsigned char* mark)
+{
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= 5 * n) return;
+    const long long i = e / 5;
+    int lo = 0, hi = nbins;   // bin: bin_off[bin] <= i < bin_off[bin + 1]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) / 2;
+        if (bin_off[mid] <= i) lo = mid;
+        else hi = mid;
+    }
+    int nx, ny, nz;
+    unpack_nearest(__float_as_uint(rec[i].q[3].w), nx, ny, nz);
+    const int y = ny - 2 + (int)(e - 5 * i);
+    if (y < 0 || y >= Gy) return;
+    unsigned char* m = mark + ((long long)lo * Gy + y) * Gz;
+    for (int z = max(nz - 2, 0); z <= min(nz + 2, Gz - 1); ++z) m[z] = 1;
+}
+
+cudaError_t launch_mark_columns(const TapRecord* rec, long long n, const long long* bin_off, int nbins, const int* G,
+                                unsigned char* mark, cudaStream_t s)
+{
+    const cudaError_t e = cudaMemsetAsync(mark, 0, (size_t)nbins * G[1] * G[2], s);
+    if (e != cudaSuccess || n == 0) return e;
+    k_mark_columns<<<(unsigned)((5 * n + 255) / 256), 256, 0, s>>>(rec, n, bin_off, nbins, G[1], G[2], mark);
+    return cudaGetLastError();
+}
+
 __global__ void k_record_nearest(const TapRecord* __restrict__ rec, long long n, unsigned* __restrict__ out)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -53,6 +53,10 @@ cudaError_t launch_tap_records(const double* k, const int* sample_idx, long long
                                TapRecord* out, cudaStream_t s);
 cudaError_t launch_interp(const InterpArgs& a, long long max_bin_samples, int nbins, int cc, cudaStream_t s);
 cudaError_t launch_spread(const SpreadArgs& a, int ntiles, int nbins, bool kahan, int wpp, cudaStream_t s);
+// mark[bin][column] (zeroed here) = 1 for the grid columns within +-2 cells of
+// some sample's nearest point
+cudaError_t launch_mark_columns(const TapRecord* rec, long long n, const long long* bin_off, int nbins, const int* G,
+                                unsigned char* mark, cudaStream_t s);
 // packed nearest grid point of each tap record
 cudaError_t launch_record_nearest(const TapRecord* rec, long long n, unsigned* out, cudaStream_t s);
 size_t spread_smem_bytes(int cc, bool kahan);
