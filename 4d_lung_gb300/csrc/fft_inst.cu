@@ -39,9 +39,11 @@ struct SizeImpl {
 
     static constexpr int NSTAGE = 2;
     using Pipe = PipeLayout<R1, R2, TB, NSTAGE>;
-    // Toeplitz x stage: the strided passes' tile width (8-column tiles, four
-    // 128-thread blocks per SM, measured 2 % slower at L = 256)
+    // Toeplitz x stage: the strided passes' tile width (8-column tiles measured
+    // the same at L = 256), two stages (three leave room for 2 blocks per SM
+    // instead of 3: 4 % slower)
     static constexpr int TBT = TB;
+    static constexpr int NST = 2;
 
     // pipelined z passes: coil tiles in flight ahead of the FFT
     static constexpr int ZNST_F = 2, ZNST_A = 2;
@@ -106,8 +108,8 @@ struct SizeImpl {
                                          (int)QuadLayout<R1, R2, TBQ_IN>::smem_bytes(L / 2));
         if constexpr (HAS_IN)
             if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_toep_x_tma<R1, R2, TBT, NSTAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)ToepLayout<R1, R2, TBT, NSTAGE>::smem_bytes(L / 2));
+                e = cudaFuncSetAttribute(k_toep_x_tma<R1, R2, TBT, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)ToepLayout<R1, R2, TBT, NST>::smem_bytes(L / 2));
         // the z extent of an image never exceeds the grid's: size for Iz = L
         if constexpr (HAS_IN && HAS_OUT) {
             if (e == cudaSuccess) e = sax_attr<2, false>();
@@ -253,26 +255,29 @@ struct SizeImpl {
         if constexpr (!HAS_IN) {
             return cudaErrorNotSupported;
         } else {
-            using Lay = ToepLayout<R1, R2, TBT, NSTAGE>;
+            using Lay = ToepLayout<R1, R2, TBT, NST>;
             a.ntb = (a.B + TBT - 1) / TBT;
             if (4 * a.in_off != L || 2 * a.Lin != L || 4 * a.out_off != L || 2 * a.Lout != L || !a.err || nsub < 1 ||
                 batch % nsub != 0 || p_bs != (long long)L * a.B)
                 return cudaErrorNotSupported;
-            CUtensorMap map, pmap;
-            int box_rows = 0, pbox_rows = 0;
+            CUtensorMap map;
+            int box_rows = 0;
             if (!encode_strided_map(&map, a, 1, batch, TBT, &box_rows)) return cudaErrorNotSupported;
-            if (!encode_spectrum_map(&pmap, P, a.B, L, batch / nsub, TBT, &pbox_rows)) return cudaErrorNotSupported;
             const size_t smem = Lay::smem_bytes(a.Lin);
             int per_sm = 0;
-            cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_toep_x_tma<R1, R2, TBT, NSTAGE>,
+            cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_toep_x_tma<R1, R2, TBT, NST>,
                                                                           Lay::NT, smem);
             if (e != cudaSuccess) return e;
-            const long long ntiles = (long long)a.ntb * batch;
-            if (ntiles <= 0) return cudaSuccess;
-            long long nblk = (long long)sm_count() * (per_sm > 0 ? per_sm : 1);
-            if (nblk > ntiles) nblk = ntiles;
-            k_toep_x_tma<R1, R2, TBT, NSTAGE><<<(unsigned)nblk, Lay::NT, smem, s>>>(a, nsub, map, pmap, ntiles,
-                                                                                   box_rows, pbox_rows);
+            const long long nstrips = (long long)a.ntb * (batch / nsub);
+            if (nstrips <= 0) return cudaSuccess;
+            const long long nblk = (long long)sm_count() * (per_sm > 0 ? per_sm : 1);
+            // sub-items of a strip that one unit takes: all of them when that leaves every
+            // block 8 units (a last wave of an eighth at most), fewer on smaller grids
+            const long long want = std::min<long long>(nsub, (8 * nblk + nstrips - 1) / nstrips);
+            const int gsub = (int)((nsub + want - 1) / want);
+            const long long nunits = nstrips * ((nsub + gsub - 1) / gsub);
+            k_toep_x_tma<R1, R2, TBT, NST><<<(unsigned)std::min(nblk, nunits), Lay::NT, smem, s>>>(a, P, nsub, gsub, map,
+                                                                                                  nunits, box_rows);
             return cudaGetLastError();
         }
     }

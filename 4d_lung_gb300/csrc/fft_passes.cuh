@@ -465,158 +465,183 @@ k_fft_strided_tma(StridedPassArgs a, const __grid_constant__ CUtensorMap tmap, l
 //            (the row it read)
 //   stage 3: thread n2: R1-point inverse DFT over k1 -> row n2 + R2 n1
 // The centring sign (-1)^k of the forward output and that of the adjoint
-// input cancel; the rows keep theirs.  A pipeline stage holds the tile's
-// rows (4-D map over the buffer) and its strip of P (3-D map [bins][L][B],
-// 4-byte elements), both fetched by the TMA unit NSTAGE - 1 tiles ahead on
-// one mbarrier.  Tiles t -> (sub-item t % nsub, column strip, bin): the nsub
-// tiles of one strip run back to back, so that the strip of P they share
-// comes from DRAM once.  Bounded waits and the timeout exit are those of
-// k_fft_strided_tma.
+// input cancel.  The rows' sign is (-1)^n2 with an even R2 (FOLD): both
+// twiddles of (n2, k1) carry it, and no element is negated on its own.
+//
+// A pipeline stage holds the tile's rows (4-D map over the buffer), fetched by
+// the TMA unit NSTAGE - 1 tiles ahead on one mbarrier.  A unit of work is one
+// column strip of a bin and gsub of its nsub sub-items; its strip of P is the
+// same for all of them and stays in the stage-2 threads' registers (thread k1
+// multiplies by P[k1 + R1 k2] only), loaded while the unit's first tile is on
+// its way.
+//
+// Bound by the issue of its FFTs (two 256-point lines per column and item) as
+// much as by DRAM.  Four bins of 12 coils at 128 x 128 x 96 on 256 x 256 x
+// 192: 5.0 GB, 0.74 ms at the copy rate.  With P staged beside the rows of
+// every tile (2 blocks of 256 threads per SM), an unpadded twiddle table and
+// every element's sign flipped on its own: 1.52 ms; this form: 1.33 ms.  3
+// stages 1.38 (2 blocks fit), 2 blocks per SM 1.37, 8-column tiles 1.33.
+// Bounded waits and the timeout exit are those of k_fft_strided_tma.
 // ---------------------------------------------------------------------------
 template <int R1, int R2, int TB, int NSTAGE>
 struct ToepLayout {
     static constexpr int L = R1 * R2;
     static constexpr int NT = TB * (R1 > R2 ? R1 : R2);
+    // padding of the exchange as in PipeLayout: 8-column tiles, every R2 rows
+    static constexpr int YP = TB == 8 ? 8 : 0;
+    static constexpr int SY = L * TB + R1 * YP;
+    static constexpr int MINB = NT <= 128 ? 6 : R2 > 16 ? 2 : 3;
+    __host__ __device__ static int stage_elems(int Lin) { return (Lin * TB + 15) & ~15; }
     static size_t smem_bytes(int Lin)
     {
-        return 1024 + (size_t)NSTAGE * Lin * TB * sizeof(float2) + (size_t)NSTAGE * L * TB * sizeof(float) +
-               (size_t)L * TB * sizeof(float2) + (size_t)L * sizeof(float2) + NSTAGE * sizeof(uint64_t);
+        return 128 + ((size_t)NSTAGE * stage_elems(Lin) + (size_t)SY + L + R2) * sizeof(float2) + NSTAGE * sizeof(uint64_t);
     }
 };
 
 template <int R1, int R2, int TB, int NSTAGE>
-__global__ void __launch_bounds__(ToepLayout<R1, R2, TB, NSTAGE>::NT, ToepLayout<R1, R2, TB, NSTAGE>::NT <= 128 ? 4 : 2)
-k_toep_x_tma(StridedPassArgs a, int nsub, const __grid_constant__ CUtensorMap tmap,
-             const __grid_constant__ CUtensorMap pmap, long long ntiles, int box_rows, int pbox_rows)
+__global__ void __launch_bounds__(ToepLayout<R1, R2, TB, NSTAGE>::NT, ToepLayout<R1, R2, TB, NSTAGE>::MINB)
+k_toep_x_tma(StridedPassArgs a, const float* __restrict__ P, int nsub, int gsub, const __grid_constant__ CUtensorMap tmap,
+             long long nunits, int box_rows)
 {
+    using Lay = ToepLayout<R1, R2, TB, NSTAGE>;
     constexpr int L = R1 * R2;
-    constexpr int NT = ToepLayout<R1, R2, TB, NSTAGE>::NT;
+    constexpr int NT = Lay::NT;
+    constexpr int YP = Lay::YP;
+    constexpr bool FOLD = R2 % 2 == 0;
     static_assert(R1 % 4 == 0, "the stored rows L/4 .. 3L/4 need R1 % 4 == 0");
     extern __shared__ float4 s_pipe[];
-    const uint32_t pad = (1024u - (smem_addr(s_pipe) & 1023u)) & 1023u;   // as in k_fft_strided_tma
-    const int stage_elems = a.Lin * TB;
+    const uint32_t pad = (128u - (smem_addr(s_pipe) & 127u)) & 127u;   // as in k_fft_strided_tma
+    const int stage_elems = Lay::stage_elems(a.Lin);
     float2* s_in = reinterpret_cast<float2*>(reinterpret_cast<char*>(s_pipe) + pad);
-    float* s_p = reinterpret_cast<float*>(s_in + (size_t)NSTAGE * stage_elems);
-    float2* s_y = reinterpret_cast<float2*>(s_p + (size_t)NSTAGE * L * TB);
-    float2* s_tw = s_y + L * TB;
-    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_tw + L);
-    __shared__ long long s_item[NSTAGE];   // per stage: the tile's batch item
-    __shared__ int s_b0[NSTAGE];           // and first column (left by the issuing thread)
+    float2* s_y = s_in + (size_t)NSTAGE * stage_elems;
+    float2* s_tw = s_y + Lay::SY;   // [n2][k1], R1 + 1 a row: W^(n2 k1), signed when FOLD
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_tw + L + R2);
     const int tid = threadIdx.x;
-    for (int m = tid; m < L; m += NT) s_tw[m] = a.tw[m];
+    for (int m = tid; m < L; m += NT) {
+        const int n2 = m / R1, k1 = m % R1;
+        const float2 w = a.tw[n2 * k1];
+        s_tw[n2 * (R1 + 1) + k1] = FOLD ? parity(w, n2) : w;
+    }
     if (tid == 0) {
         for (int s = 0; s < NSTAGE; ++s) mbar_init(&s_bar[s], 1);
         fence_mbar_init();
     }
     __syncthreads();
-    const long long my_n = ntiles > (long long)blockIdx.x ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    const int ngrp = (nsub + gsub - 1) / gsub;
 
-    auto decode = [&](long long t, long long& item, long long& bin, int& b0) {
-        const long long strip = t / nsub;
-        const int sub = (int)(t - strip * nsub);
+    // thread 0's cursor: the next tile to fetch
+    long long iu = blockIdx.x, ibin = 0;
+    int isub = 0, iend = 0, ib0 = 0;
+    long long ik = 0;
+    auto unit = [&](long long un, long long& bin, int& b0, int& s0, int& s1) {
+        const long long strip = un / ngrp;
+        s0 = (int)(un - strip * ngrp) * gsub;
+        s1 = s0 + gsub < nsub ? s0 + gsub : nsub;
         bin = strip / a.ntb;
         b0 = (int)(strip - bin * a.ntb) * TB;
-        item = bin * nsub + sub;
     };
-    auto issue = [&](long long k) {   // thread 0 only
-        const long long t = blockIdx.x + k * gridDim.x;
-        long long item, bin;
-        int b0;
-        decode(t, item, bin, b0);
-        const int s = (int)(k % NSTAGE);
-        s_item[s] = item;
-        s_b0[s] = b0;
-        mbar_arrive_expect_tx(&s_bar[s], (uint32_t)(stage_elems * sizeof(float2) + L * TB * sizeof(float)));
+    auto issue = [&]() {   // thread 0 only; nothing past the last unit
+        if (isub == iend) {
+            if (iu >= nunits) return;
+            unit(iu, ibin, ib0, isub, iend);
+            iu += gridDim.x;
+        }
+        const int s = (int)(ik % NSTAGE);
+        mbar_arrive_expect_tx(&s_bar[s], (uint32_t)(a.Lin * TB * sizeof(float2)));
         float2* dst = s_in + (size_t)s * stage_elems;
         for (int r0 = 0; r0 < a.Lin; r0 += box_rows)
-            tma_load_4d(dst + (size_t)r0 * TB, &tmap, b0, r0, 0, (int)item, &s_bar[s]);
-        float* pdst = s_p + (size_t)s * L * TB;
-        for (int r0 = 0; r0 < L; r0 += pbox_rows) tma_load_3d(pdst + (size_t)r0 * TB, &pmap, b0, r0, (int)bin, &s_bar[s]);
+            tma_load_4d(dst + (size_t)r0 * TB, &tmap, ib0, r0, 0, (int)(ibin * nsub + isub), &s_bar[s]);
+        ++isub;
+        ++ik;
     };
 
     if (tid == 0)
-        for (long long k = 0; k < NSTAGE - 1 && k < my_n; ++k) issue(k);
-    for (long long k = 0; k < my_n; ++k) {
-        const int s = (int)(k % NSTAGE);
-        if (tid == 0 && k + NSTAGE - 1 < my_n) issue(k + NSTAGE - 1);
-        const bool ok = mbar_wait_bounded(&s_bar[s], (uint32_t)((k / NSTAGE) & 1), PIPE_WAIT_NS);
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) {
-                atomicExch(a.err, 1);
-                for (long long j = k; j < my_n && j < k + NSTAGE; ++j)
-                    mbar_wait_bounded(&s_bar[j % NSTAGE], (uint32_t)((j / NSTAGE) & 1), PIPE_WAIT_NS);
-            }
-            return;
-        }
-        // the tile's coordinates, as the issuing thread decoded them (no
-        // per-thread 64-bit divisions)
-        const long long item = s_item[s];
-        const int b0 = s_b0[s];
-        const int bi = tid % TB;
+        for (int j = 0; j < NSTAGE - 1; ++j) issue();
+    long long k = 0;
+    const int bi = tid % TB, row = tid / TB;   // row: n2 in stages 1 and 3, k1 in stage 2
+    for (long long un = blockIdx.x; un < nunits; un += gridDim.x) {
+        long long bin;
+        int b0, sub, sub1;
+        unit(un, bin, b0, sub, sub1);
         const int b = b0 + bi;
         const bool bok = b < a.B;
-        const float2* sin_s = s_in + (size_t)s * stage_elems;
-        const float* sp = s_p + (size_t)s * L * TB;
+        float pv[R2];
         {
-            const int n2 = tid / TB;
-            if (n2 < R2) {
+            const float* pp = P + (bin * L + row) * a.B + b;
+#pragma unroll
+            for (int k2 = 0; k2 < R2; ++k2) pv[k2] = row < R1 && bok ? __ldg(pp + (long long)(R1 * k2) * a.B) : 0.f;
+        }
+        float2* out = a.out + (bin * nsub + sub) * a.out_bs + (long long)row * a.B + b;
+        for (; sub < sub1; ++sub, ++k, out += a.out_bs) {
+            const int s = (int)(k % NSTAGE);
+            if (tid == 0) issue();
+            const bool ok = mbar_wait_bounded(&s_bar[s], (uint32_t)((k / NSTAGE) & 1), PIPE_WAIT_NS);
+            if (__syncthreads_or(!ok)) {
+                if (tid == 0) {
+                    atomicExch(a.err, 1);
+                    for (long long j = k; j < ik; ++j)
+                        mbar_wait_bounded(&s_bar[j % NSTAGE], (uint32_t)((j / NSTAGE) & 1), PIPE_WAIT_NS);
+                }
+                return;
+            }
+            if (row < R2) {
                 float2 v[R1];
-                const float2* src = sin_s + n2 * TB + bi;
+                const float2* src = s_in + (size_t)s * stage_elems + row * TB + bi;
 #pragma unroll
                 for (int n1 = 0; n1 < R1; ++n1) {
-                    if (n1 >= R1 / 4 && n1 < 3 * R1 / 4)
-                        v[n1] = parity(src[(R2 * (n1 - R1 / 4)) * TB], R2 * n1 + n2);
-                    else
+                    if (n1 >= R1 / 4 && n1 < 3 * R1 / 4) {
+                        const float2 x = src[(R2 * (n1 - R1 / 4)) * TB];
+                        v[n1] = FOLD ? x : parity(x, R2 * n1 + row);
+                    } else {
                         v[n1] = make_float2(0.f, 0.f);
+                    }
                 }
                 DftMid<R1, -1>::run(v);
 #pragma unroll
                 for (int q = 0; q < R1; ++q) {
                     float2 tv = v[q];
-                    if (q > 0) tv = table_twiddle<-1>(tv, s_tw[n2 * q]);
-                    s_y[(q * R2 + n2) * TB + bi] = tv;
+                    if (FOLD || q > 0) tv = table_twiddle<-1>(tv, s_tw[row * (R1 + 1) + q]);
+                    s_y[(q * R2 + row) * TB + bi + q * YP] = tv;
                 }
             }
-        }
-        __syncthreads();
-        const int k1 = tid / TB;
-        float2 u[R2];
-        if (k1 < R1) {
+            __syncthreads();
+            if (row < R1) {
+                float2* y = s_y + row * (R2 * TB + YP) + bi;
+                const float2* w = s_tw + row;
+                float2 u[R2];
 #pragma unroll
-            for (int n2 = 0; n2 < R2; ++n2) u[n2] = s_y[(k1 * R2 + n2) * TB + bi];
-            Dft<R2, -1>::run(u);
+                for (int n2 = 0; n2 < R2; ++n2) u[n2] = y[n2 * TB];
+                Dft<R2, -1>::run(u);
 #pragma unroll
-            for (int k2 = 0; k2 < R2; ++k2) {
-                const float pv = sp[(k1 + R1 * k2) * TB + bi];
-                u[k2].x *= pv;
-                u[k2].y *= pv;
+                for (int k2 = 0; k2 < R2; ++k2) {
+                    u[k2].x *= pv[k2];
+                    u[k2].y *= pv[k2];
+                }
+                Dft<R2, +1>::run(u);
+                // back into the positions this thread read (row k1): no other
+                // thread touches them before the barrier
+#pragma unroll
+                for (int n2 = 0; n2 < R2; ++n2)
+                    y[n2 * TB] = n2 > 0 ? table_twiddle<+1>(u[n2], w[n2 * (R1 + 1)]) : u[n2];
             }
-            Dft<R2, +1>::run(u);
-            // back into the positions this thread read (row k1): no other
-            // thread touches them before the barrier
-#pragma unroll
-            for (int n2 = 0; n2 < R2; ++n2)
-                s_y[(k1 * R2 + n2) * TB + bi] = n2 > 0 ? table_twiddle<+1>(u[n2], s_tw[n2 * k1]) : u[n2];
-        }
-        __syncthreads();
-        {
-            const int n2 = tid / TB;
-            if (n2 < R2) {
+            __syncthreads();
+            if (row < R2) {
                 float2 w[R1];
 #pragma unroll
-                for (int q = 0; q < R1; ++q) w[q] = s_y[(q * R2 + n2) * TB + bi];
+                for (int q = 0; q < R1; ++q) w[q] = s_y[(q * R2 + row) * TB + bi + q * YP];
                 Dft<R1, +1>::run(w);
                 if (bok) {
-                    float2* out = a.out + item * a.out_bs + b;
 #pragma unroll
-                    for (int n1 = R1 / 4; n1 < 3 * R1 / 4; ++n1)
-                        out[(long long)(n2 + R2 * (n1 - R1 / 4)) * a.B] = parity(w[n1], n2 + R2 * n1);
+                    for (int n1 = R1 / 4; n1 < 3 * R1 / 4; ++n1) {
+                        const float2 x = w[n1];
+                        out[(long long)(R2 * (n1 - R1 / 4)) * a.B] = FOLD ? x : parity(x, row + R2 * n1);
+                    }
                 }
             }
+            // no barrier here: stage 3 of thread (n2, bi) read exactly the s_y
+            // positions that its own stage 1 of the next tile writes, and the
+            // stage refilled next was last read before the barriers above
         }
-        // no barrier here: stage 3 of thread (n2, bi) read exactly the s_y
-        // positions that its own stage 1 of the next tile writes, and the
-        // stage refilled next was last read before the barrier above
     }
 }
 

@@ -18,9 +18,6 @@ cudaError_t fft_init_all();
 // promo: L2 promotion of the box's rows in bytes (64, 128 or 256)
 bool encode_strided_map(CUtensorMap* map, const StridedPassArgs& a, int A, int batch, int TB, int* box_rows,
                         int promo = 256);
-// 3-D tensor map [nbins][L][B] of 4-byte spectrum values with a TB x
-// box_rows box; false when the buffer or pitch is not 16-byte aligned
-bool encode_spectrum_map(CUtensorMap* map, const float* P, long long B, int L, int nbins, int TB, int* box_rows);
 // 4-D map [items][1][Lin][B] with a TB x box_rows box (rows past Lin read 0)
 bool encode_items_map(CUtensorMap* map, const float2* in, int B, int Lin, long long item_stride, long long items,
                       int TB, int box_rows, int promo);

@@ -76,16 +76,6 @@ CGS_D void tma_load_4d(void* dst_smem, const void* tmap, int c0, int c1, int c2,
         : "memory");
 }
 
-// 3-D tensor-map tile load (TMA) into shared memory, completion on `bar`.
-CGS_D void tma_load_3d(void* dst_smem, const void* tmap, int c0, int c1, int c2, uint64_t* bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            smem_addr(dst_smem)),
-        "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(smem_addr(bar))
-        : "memory");
-}
-
 // 4-D tensor-map tile store (TMA) from shared memory, tracked by the
 // thread's bulk async-group (commit with bulk_commit, wait with
 // bulk_wait_read / bulk_wait_all).  The shared-memory writes it reads must be

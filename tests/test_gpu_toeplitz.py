@@ -274,3 +274,26 @@ def test_toeplitz_spectrum_methods(gpu_lib, cgs, oracle_mod, img, grid, nch, ns)
         assert rel_l2(q0[b], q1[b]) < 1e-5
         assert rel_l2(q0[b], ref) < 2e-5 and rel_l2(q1[b], ref) < 2e-5
     r.close()
+
+
+# units of the fused x stage: a unit is one column strip and several coils of
+# it, all of them on large grids, one on small ones, with a short last unit
+# between; x lines with 8- and 16-column tiles.  Tolerance: fused vs unfused
+# x stage, as above.
+@pytest.mark.parametrize("img,grid,nch,nb", [
+    ((16, 96, 96), (32, 192, 192), 3, 4),     # 9216 strips: whole strips
+    ((16, 96, 96), (32, 192, 192), 3, 2),     # 4608 strips: two coils, then one
+    ((16, 64, 48), (32, 128, 96), 7, 3),      # 2304 strips: two coils at a time, one left
+    ((160, 8, 8), (320, 16, 16), 5, 1),       # 16 x 20, 8-column tiles
+    ((10, 20, 10), (20, 40, 20), 3, 2),       # 4 x 5: signs element by element
+])
+def test_toeplitz_units_of_the_fused_stage(gpu_lib, cgs, img, grid, nch, nb):
+    k, dcf, S, bins, x = random_case(img, nch, 300, nb, seed=9)
+    r = make_reco(cgs, img, grid, nch, k, dcf, S, bins)
+    r.set_toeplitz(1)
+    q1, n1 = apply(r, x)
+    r.set_toeplitz(2)
+    q2, n2 = apply(r, x)
+    assert n1 == 5 and n2 == 7
+    for b in range(nb):
+        assert rel_l2(q1[b], q2[b]) < 1e-6
