@@ -119,15 +119,25 @@ struct SizeImpl {
             if (e == cudaSuccess) e = sax_attr<6, false>();
             if (e == cudaSuccess) e = sax_attr<6, true>();
         }
+        if (e == cudaSuccess) e = z_attr<false>();
+        if constexpr (HAS_OUT)
+            if (e == cudaSuccess) e = z_attr<true>();
+        return e;
+    }
+
+    template <bool HALF>
+    static cudaError_t z_attr()
+    {
+        cudaError_t e = cudaFuncSetAttribute(k_fwd_z_pipe<R1, R2, LPB, ZNST_F, false, HALF>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)ZF::smem_bytes(HALF ? L / 2 : L, false, HALF));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_fwd_z_pipe<R1, R2, LPB, ZNST_F, false>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZF::smem_bytes(L, false));
+            e = cudaFuncSetAttribute(k_fwd_z_pipe<R1, R2, LPB, ZNST_F, true, HALF>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)ZF::smem_bytes(HALF ? L / 2 : L, false, HALF));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_fwd_z_pipe<R1, R2, LPB, ZNST_F, true>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZF::smem_bytes(L, false));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_adj_z_pipe<R1, R2, LPB, ZNST_A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)ZA::smem_bytes(L, true));
+            e = cudaFuncSetAttribute(k_adj_z_pipe<R1, R2, LPB, ZNST_A, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)ZA::smem_bytes(HALF ? L / 2 : L, true, HALF));
         return e;
     }
 
@@ -333,6 +343,8 @@ struct SizeImpl {
         else k_fft_contig<R1, R2, +1, LPB><<<grid, NT_C, 0, s>>>(a);
         return cudaGetLastError();
     }
+    // the image is the middle half of the line
+    static bool half_line(int lo, int I) { return 4 * lo == L && 2 * I == L; }
     // z passes: one block per (line block, batch item), items fastest (zp_item)
     static cudaError_t fwd_z(const FwdZArgs& a0, int batch, cudaStream_t s)
     {
@@ -342,8 +354,16 @@ struct SizeImpl {
         // bulk copies need 16-byte aligned tiles: even Iz and coil strides
         if (a.err && a.smaps && a.x_cs == 0 && a.Iz <= L && (a.Iz & 1) == 0 && (a.coil_in & 1) == 0 &&
             al16(a.smaps)) {
-            if (a.cg) k_fwd_z_pipe<R1, R2, LPB, ZNST_F, true><<<grid, NT_C, ZF::smem_bytes(a.Iz, false), s>>>(a);
-            else k_fwd_z_pipe<R1, R2, LPB, ZNST_F, false><<<grid, NT_C, ZF::smem_bytes(a.Iz, false), s>>>(a);
+            if constexpr (HAS_OUT)
+                if (half_line(a.lo_z, a.Iz)) {
+                    const size_t smem = ZF::smem_bytes(a.Iz, false, true);
+                    if (a.cg) k_fwd_z_pipe<R1, R2, LPB, ZNST_F, true, true><<<grid, NT_C, smem, s>>>(a);
+                    else k_fwd_z_pipe<R1, R2, LPB, ZNST_F, false, true><<<grid, NT_C, smem, s>>>(a);
+                    return cudaGetLastError();
+                }
+            const size_t smem = ZF::smem_bytes(a.Iz, false, false);
+            if (a.cg) k_fwd_z_pipe<R1, R2, LPB, ZNST_F, true, false><<<grid, NT_C, smem, s>>>(a);
+            else k_fwd_z_pipe<R1, R2, LPB, ZNST_F, false, false><<<grid, NT_C, smem, s>>>(a);
             return cudaGetLastError();
         }
         if (a.cg) k_fwd_z<R1, R2, LPB, true><<<grid, NT_C, 0, s>>>(a);
@@ -358,7 +378,12 @@ struct SizeImpl {
         dim3 grid((unsigned)((long long)adj_blocks(a.nl) * batch));
         if (a.err && a.smaps && a.Iz <= L && (a.Iz & 1) == 0 && (a.coil_s & 1) == 0 && (a.coil_in & 1) == 0 &&
             (a.in_bs & 1) == 0 && al16(a.smaps) && al16(a.in)) {
-            k_adj_z_pipe<R1, R2, LPB, ZNST_A><<<grid, NT_C, ZA::smem_bytes(a.Iz, true), s>>>(a);
+            if constexpr (HAS_OUT)
+                if (half_line(a.lo_z, a.Iz)) {
+                    k_adj_z_pipe<R1, R2, LPB, ZNST_A, true><<<grid, NT_C, ZA::smem_bytes(a.Iz, true, true), s>>>(a);
+                    return cudaGetLastError();
+                }
+            k_adj_z_pipe<R1, R2, LPB, ZNST_A, false><<<grid, NT_C, ZA::smem_bytes(a.Iz, true, false), s>>>(a);
             return cudaGetLastError();
         }
         k_adj_z<R1, R2, LPB><<<grid, NT_C, 0, s>>>(a);

@@ -78,20 +78,22 @@ CGS_D FwdZCg fwd_z_cg(const FwdZArgs& a, int item)
 // eb: element index of the line start within the batch.
 constexpr int fwd_z_group(int r1) { return r1 % 8 == 0 ? 8 : (r1 % 4 == 0 ? 4 : (r1 % 2 == 0 ? 2 : 1)); }
 
-template <int R1, int R2, class Put>
+template <int R1, int R2, bool HALF, class Put>
 CGS_D void fwd_z_fused_line(const FwdZArgs& a, const FwdZCg& u, long long eb, int n2, float axy, Put put)
 {
-    constexpr int GRP = fwd_z_group(R1);
+    // HALF: the image is the line's middle half, n1 in [R1/4, 3R1/4); groups
+    // of 4, as the caller keeps the results in registers
+    constexpr int GRP = HALF ? (R1 / 2 < 4 ? R1 / 2 : 4) : fwd_z_group(R1);
     float2* __restrict__ P = a.cg_p + eb;
     const float2* __restrict__ Rr = a.cg_r + eb;
     float2* __restrict__ X = a.cg_x + eb;
 #pragma unroll
-    for (int g0 = 0; g0 < R1; g0 += GRP) {
+    for (int g0 = HALF ? R1 / 4 : 0; g0 < (HALF ? 3 * R1 / 4 : R1); g0 += GRP) {
         float2 pv[GRP], rv[GRP], xv[GRP];
 #pragma unroll
         for (int j = 0; j < GRP; ++j) {
-            const int zi = R2 * (g0 + j) + n2 - a.lo_z;
-            if (zi >= 0 && zi < a.Iz) {
+            const int zi = HALF ? R2 * (g0 + j - R1 / 4) + n2 : R2 * (g0 + j) + n2 - a.lo_z;
+            if (HALF || (zi >= 0 && zi < a.Iz)) {
                 pv[j] = P[zi];
                 rv[j] = Rr[zi];
                 xv[j] = X[zi];
@@ -101,8 +103,8 @@ CGS_D void fwd_z_fused_line(const FwdZArgs& a, const FwdZCg& u, long long eb, in
         for (int j = 0; j < GRP; ++j) {
             const int n1 = g0 + j;
             const int l = R2 * n1 + n2;
-            const int zi = l - a.lo_z;
-            if (zi >= 0 && zi < a.Iz) {
+            const int zi = HALF ? R2 * (n1 - R1 / 4) + n2 : l - a.lo_z;
+            if (HALF || (zi >= 0 && zi < a.Iz)) {
                 X[zi] = cg_axpy(xv[j], u.ar, u.ai, pv[j]);
                 const float2 p1 = cg_axpy(rv[j], u.br, u.bi, pv[j]);
                 P[zi] = p1;
@@ -762,7 +764,7 @@ k_fwd_z(FwdZArgs a)
                 if (CGF && cg.upd) {
 #pragma unroll
                     for (int n1 = 0; n1 < R1; ++n1) xa[n1] = make_float2(0.f, 0.f);
-                    fwd_z_fused_line<R1, R2>(a, cg, eb, n2, axy, [&](int n1, int, float2 v) { xa[n1] = v; });
+                    fwd_z_fused_line<R1, R2, false>(a, cg, eb, n2, axy, [&](int n1, int, float2 v) { xa[n1] = v; });
                 } else {
                     const float2* xl = a.x + eb;
 #pragma unroll
@@ -950,7 +952,21 @@ k_adj_z(AdjZArgs a)
 // shared-memory stages, NST - 1 coils ahead of the FFT.  Arithmetic and
 // results are those of k_fwd_z / k_adj_z.  Every wait is bounded (2 s); on a
 // timeout the block sets *err, lets its issued copies land and exits.
-// Shared layout: [NST stages][bars][twiddles][exchange rows].
+// Shared layout: [NST stages][twiddles][exchange rows][image lines][bars].
+//
+// The centring signs of a line's two ends are (-1)^n2 and (-1)^k1 with even
+// splits: the twiddles W^(n2 k1) carry them.  HALF: the image is the middle half
+// of the line (two-fold oversampling, R2 % 4 == 0): its rows are known at compile
+// time, n1 in [R1/4, 3R1/4) forward and k2 in [R2/4, 3R2/4) adjoint, so half of
+// the loads, products and codelet work on zeros or unused rows is not done,
+// and the forward pass keeps its image values in registers (4 blocks of 256
+// threads per SM instead of 3).
+//
+// 16 bins, 12 coils, 128 x 128 lines of 96 -> 192: forward 5.1 GB, 0.76 ms at the
+// copy rate, and adjoint 5.2 GB, 0.76 ms; both issue-bound before they are
+// DRAM-bound.  Forward 1.25 -> 0.92 ms (3 blocks per SM 0.97), adjoint 1.27 ->
+// 0.96 ms (1.11 before its twiddles stayed in registers and a barrier per coil
+// fell away).  160 x 160 lines of 112 -> 224: 0.21 -> 0.19 and 0.32 -> 0.24 ms.
 // ---------------------------------------------------------------------------
 template <int R1, int R2, int LPB, int NST>
 struct ZPipeLayout {
@@ -963,9 +979,9 @@ struct ZPipeLayout {
     // twiddles W^(n2 k1) as R2 rows of R1 + 1 (padded: a warp's rows in
     // different banks)
     static constexpr int TW = R2 * (R1 + 1);
-    static size_t smem_bytes(int Iz, bool adj)
+    static size_t smem_bytes(int Iz, bool adj, bool half)
     {
-        return (NST * stage_elems(Iz, adj) + TW + (size_t)LPB * Lay::LINE + (adj ? 0 : (size_t)LPB * Iz)) *
+        return (NST * stage_elems(Iz, adj) + TW + (size_t)LPB * Lay::LINE + (adj || half ? 0 : (size_t)LPB * Iz)) *
                    sizeof(float2) +
                16 * NST;
     }
@@ -973,25 +989,26 @@ struct ZPipeLayout {
 
 // CGF: the fused CG form (a.cg set); a separate instantiation, so that the
 // plain pass compiles without the update path.
-template <int R1, int R2, int LPB, int NST, bool CGF>
-__global__ void __launch_bounds__(LPB * ContigLayout<R1, R2>::RMAX, (R1 > 16 || R2 > 16) ? 2 : 3)
+template <int R1, int R2, int LPB, int NST, bool CGF, bool HALF>
+__global__ void __launch_bounds__(LPB * ContigLayout<R1, R2>::RMAX, (R1 > 16 || R2 > 16) ? 2 : HALF ? 4 : 3)
 k_fwd_z_pipe(FwdZArgs a)
 {
     using Lay = ContigLayout<R1, R2>;
     using ZL = ZPipeLayout<R1, R2, LPB, NST>;
     constexpr int L = Lay::L;
     constexpr int SIGN = -1;
+    static_assert(R1 % 4 == 0, "the folded output sign and the half-line form");
     extern __shared__ float4 s_dyn[];
     const size_t se = ZL::stage_elems(a.Iz, false);
     float2* s_stage = reinterpret_cast<float2*>(s_dyn);
     float2* s_tw = s_stage + NST * se;      // [R2][R1 + 1]: W^(n2 k1)
     float2* s_y = s_tw + ZL::TW;
-    float2* s_xa = s_y + LPB * Lay::LINE;   // x * apod * parity of the block's lines, [LPB][Iz]
-    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_xa + (size_t)LPB * a.Iz);
+    float2* s_xa = s_y + LPB * Lay::LINE;   // not HALF: x * apod * parity of the block's lines, [LPB][Iz]
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_xa + (HALF ? 0 : (size_t)LPB * a.Iz));
     const int tid = threadIdx.x;
     for (int m = tid; m < L; m += ZL::NT) {
         const int r = m / R1, q = m - r * R1;
-        s_tw[r * (R1 + 1) + q] = a.tw[r * q];
+        s_tw[r * (R1 + 1) + q] = parity(a.tw[r * q], q);   // (-1)^k1 of the output rows k1 + R1 k2
     }
     const int item = zp_item(a.nbatch);
     const long long line0 = zp_lblk(a.nbatch) * LPB;
@@ -1016,20 +1033,32 @@ k_fwd_z_pipe(FwdZArgs a)
     const long long line1 = line0 + ln1;
     const bool act1 = ln1 < LPB && line1 < a.nl;
     float2* xa = s_xa + (size_t)ln1 * a.Iz;   // written and read by this thread only
+    float2 xr[HALF ? R1 / 2 : 1];             // HALF: the same values, of n1 = R1 / 4 + j
     if (act1) {
         const int ix = (int)(line1 / a.Iy), iy = (int)(line1 - (long long)ix * a.Iy);
         const float axy = a.apx[ix] * a.apy[iy];
         const FwdZCg cg = CGF ? fwd_z_cg(a, item) : FwdZCg{false, 0.f, 0.f, 0.f, 0.f};
         const long long eb = (long long)item * a.x_bs + line1 * a.Iz;
         if (CGF && cg.upd) {
-            fwd_z_fused_line<R1, R2>(a, cg, eb, n2, axy, [&](int, int zi, float2 v) { xa[zi] = v; });
+            fwd_z_fused_line<R1, R2, HALF>(a, cg, eb, n2, axy, [&](int n1, int zi, float2 v) {
+                if constexpr (HALF) xr[n1 - R1 / 4] = v;
+                else xa[zi] = v;
+            });
         } else {
             const float2* xl = a.x + eb;
+            if constexpr (HALF) {
 #pragma unroll
-            for (int n1 = 0; n1 < R1; ++n1) {
-                const int l = R2 * n1 + n2;
-                const int zi = l - a.lo_z;
-                if (zi >= 0 && zi < a.Iz) xa[zi] = parity(cscale(xl[zi], axy * a.apz[zi]), l);
+                for (int j = 0; j < R1 / 2; ++j) {
+                    const int zi = R2 * j + n2;
+                    xr[j] = parity(cscale(xl[zi], axy * a.apz[zi]), R2 * (j + R1 / 4) + n2);
+                }
+            } else {
+#pragma unroll
+                for (int n1 = 0; n1 < R1; ++n1) {
+                    const int l = R2 * n1 + n2;
+                    const int zi = l - a.lo_z;
+                    if (zi >= 0 && zi < a.Iz) xa[zi] = parity(cscale(xl[zi], axy * a.apz[zi]), l);
+                }
             }
         }
     }
@@ -1037,6 +1066,14 @@ k_fwd_z_pipe(FwdZArgs a)
     const long long line2 = line0 + ln2;
     const bool act2 = ln2 < LPB && line2 < a.nl;
 
+    // the thread's twiddles, the same for every coil, where the registers allow
+    // (lines of 192 measured 5 % slower with them: spills at 4 blocks per SM)
+    constexpr bool TWR = R1 > 16 || R2 > 16;
+    float2 twr[TWR ? R1 : 1];
+    if constexpr (TWR) {
+#pragma unroll
+        for (int kk = 1; kk < R1; ++kk) twr[kk] = s_tw[n2 * (R1 + 1) + kk];
+    }
     for (int c = 0; c < a.nch; ++c) {
         const int st = c % NST;
         // stage (c - 1) % NST was last read in stage 1 of coil c - 1, before
@@ -1056,14 +1093,21 @@ k_fwd_z_pipe(FwdZArgs a)
             float2 v[R1];
 #pragma unroll
             for (int n1 = 0; n1 < R1; ++n1) {
-                const int zi = R2 * n1 + n2 - a.lo_z;
-                v[n1] = (zi >= 0 && zi < a.Iz) ? cmul(xa[zi], S[zi]) : make_float2(0.f, 0.f);
+                if constexpr (HALF) {
+                    v[n1] = n1 >= R1 / 4 && n1 < 3 * R1 / 4
+                                ? cmul(xr[(n1 - R1 / 4) & (R1 / 2 - 1)], S[R2 * (n1 - R1 / 4) + n2])
+                                : make_float2(0.f, 0.f);
+                } else {
+                    const int zi = R2 * n1 + n2 - a.lo_z;
+                    v[n1] = (zi >= 0 && zi < a.Iz) ? cmul(xa[zi], S[zi]) : make_float2(0.f, 0.f);
+                }
             }
-            Dft<R1, SIGN>::run(v);
+            if constexpr (HALF) DftMid<R1, SIGN>::run(v);
+            else Dft<R1, SIGN>::run(v);
 #pragma unroll
             for (int kk = 0; kk < R1; ++kk) {
                 float2 t = v[kk];
-                if (kk > 0) t = table_twiddle<SIGN>(t, s_tw[n2 * (R1 + 1) + kk]);
+                if (kk > 0) t = table_twiddle<SIGN>(t, TWR ? twr[TWR ? kk : 0] : s_tw[n2 * (R1 + 1) + kk]);
                 s_y[ln1 * Lay::LINE + n2 * Lay::R1P + kk] = t;
             }
         }
@@ -1075,15 +1119,12 @@ k_fwd_z_pipe(FwdZArgs a)
             Dft<R2, SIGN>::run(u);
             float2* o = outb + (long long)c * a.coil_out + line2 * L;
 #pragma unroll
-            for (int k2 = 0; k2 < R2; ++k2) {
-                const int l = k1 + R1 * k2;
-                o[l] = parity(u[k2], l);
-            }
+            for (int k2 = 0; k2 < R2; ++k2) o[k1 + R1 * k2] = u[k2];
         }
     }
 }
 
-template <int R1, int R2, int LPB, int NST>
+template <int R1, int R2, int LPB, int NST, bool HALF>
 __global__ void __launch_bounds__(LPB * ContigLayout<R1, R2>::RMAX)
 k_adj_z_pipe(AdjZArgs a)
 {
@@ -1091,6 +1132,9 @@ k_adj_z_pipe(AdjZArgs a)
     using ZL = ZPipeLayout<R1, R2, LPB, NST>;
     constexpr int L = Lay::L;
     constexpr int SIGN = +1;
+    constexpr bool INF = R2 % 2 == 0;   // the input rows' sign is (-1)^n2
+    static_assert(R1 % 2 == 0, "the folded output sign");
+    static_assert(!HALF || R2 % 4 == 0, "the half-line form");
     constexpr int NT = ZL::NT;
     extern __shared__ float4 s_dyn[];
     __shared__ double s_red[2][NT / 32];
@@ -1103,7 +1147,7 @@ k_adj_z_pipe(AdjZArgs a)
     const int tid = threadIdx.x;
     for (int m = tid; m < L; m += NT) {
         const int r = m / R1, q = m - r * R1;
-        s_tw[r * (R1 + 1) + q] = a.tw[r * q];
+        s_tw[r * (R1 + 1) + q] = parity(a.tw[r * q], INF ? r + q : q);
     }
     const int item = zp_item(a.nbatch);
     const long long lblk = zp_lblk(a.nbatch);
@@ -1136,24 +1180,29 @@ k_adj_z_pipe(AdjZArgs a)
     const long long line2 = line0 + ln2;
     const bool act2 = ln2 < LPB && line2 < a.nl;
 
-    float2 acc[R2];
+    // rows k1 + R1 k2 of the image: k2 in [K0, K1)
+    constexpr int K0 = HALF ? R2 / 4 : 0, K1 = HALF ? 3 * R2 / 4 : R2;
+    float2 acc[K1 - K0];
 #pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) acc[k2] = make_float2(0.f, 0.f);
+    for (int j = 0; j < K1 - K0; ++j) acc[j] = make_float2(0.f, 0.f);
 
+    float2 twr[R1];   // the thread's twiddles, the same for every coil
+#pragma unroll
+    for (int kk = 1; kk < R1; ++kk) twr[kk] = s_tw[n2 * (R1 + 1) + kk];
     for (int c = 0; c < a.nch; ++c) {
         const int st = c % NST;
-        // stage (c - 1) % NST is read up to stage 2 of coil c - 1
-        __syncthreads();
-        if (tid == 0 && c + NST - 1 < a.nch) issue(c + NST - 1);
         const bool ok = mbar_wait_bounded(&s_bar[st], (uint32_t)((c / NST) & 1), PIPE_WAIT_NS);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) {
                 atomicExch(a.err, 1);
-                for (int j = c; j < a.nch && j < c + NST; ++j)
+                for (int j = c; j < a.nch && j < c + NST - 1; ++j)
                     mbar_wait_bounded(&s_bar[j % NST], (uint32_t)((j / NST) & 1), PIPE_WAIT_NS);
             }
             return;
         }
+        // stage (c - 1) % NST was last read in stage 2 of coil c - 1, before the
+        // barrier above
+        if (tid == 0 && c + NST - 1 < a.nch) issue(c + NST - 1);
         const float2* tin = s_stage + (size_t)st * se;
         if (act1) {
             const float2* src = tin + ln1 * L;
@@ -1161,13 +1210,14 @@ k_adj_z_pipe(AdjZArgs a)
 #pragma unroll
             for (int n1 = 0; n1 < R1; ++n1) {
                 const int l = R2 * n1 + n2;
-                v[n1] = parity(src[l], l);
+                v[n1] = INF ? src[l] : parity(src[l], l);
             }
             Dft<R1, SIGN>::run(v);
 #pragma unroll
             for (int kk = 0; kk < R1; ++kk) {
                 float2 t = v[kk];
-                if (kk > 0) t = table_twiddle<SIGN>(t, s_tw[n2 * (R1 + 1) + kk]);
+                if (kk > 0) t = table_twiddle<SIGN>(t, twr[kk]);
+                else if (INF) t = parity(t, n2);
                 s_y[ln1 * Lay::LINE + n2 * Lay::R1P + kk] = t;
             }
         }
@@ -1179,10 +1229,9 @@ k_adj_z_pipe(AdjZArgs a)
             Dft<R2, SIGN>::run(u);
             const float2* S = tin + s_off + ln2 * a.Iz;
 #pragma unroll
-            for (int k2 = 0; k2 < R2; ++k2) {
-                const int l = k1 + R1 * k2;
-                const int zi = l - a.lo_z;
-                if (zi >= 0 && zi < a.Iz) acc[k2] = cadd(acc[k2], cmulc(parity(u[k2], l), S[zi]));
+            for (int k2 = K0; k2 < K1; ++k2) {
+                const int zi = HALF ? k1 + R1 * (k2 - K0) : k1 + R1 * k2 - a.lo_z;
+                if (HALF || (zi >= 0 && zi < a.Iz)) acc[k2 - K0] = cadd(acc[k2 - K0], cmulc(u[k2], S[zi]));
             }
         }
     }
@@ -1193,10 +1242,10 @@ k_adj_z_pipe(AdjZArgs a)
         const float sxy = a.scale * a.apx[ix] * a.apy[iy];
         float fre = 0.f, fim = 0.f;
 #pragma unroll
-        for (int k2 = 0; k2 < R2; ++k2) {
-            const int zi = k1 + R1 * k2 - a.lo_z;
-            if (zi >= 0 && zi < a.Iz) {
-                const float2 qv = cscale(acc[k2], sxy * a.apz[zi]);
+        for (int k2 = K0; k2 < K1; ++k2) {
+            const int zi = HALF ? k1 + R1 * (k2 - K0) : k1 + R1 * k2 - a.lo_z;
+            if (HALF || (zi >= 0 && zi < a.Iz)) {
+                const float2 qv = cscale(acc[k2 - K0], sxy * a.apz[zi]);
                 qb[line2 * a.Iz + zi] = qv;
                 if (a.p) {
                     const float2 pv = a.p[(long long)item * a.q_bs + line2 * a.Iz + zi];
