@@ -13,6 +13,7 @@
 // loss partials and dL/dk.
 #include "launch.h"
 #include "gridding_common.cuh"
+#include "ptx_async.cuh"
 
 #include <algorithm>
 
@@ -168,38 +169,52 @@ __global__ void __launch_bounds__(128) k_interp_grad(InterpGradArgs a)
 // one coil of the quad each, so that a warp's load of one tap takes one
 // 32-byte sector per sample.  A lane adds its coil's value and derivatives
 // over the taps in the order of the kernels above with the same products and
-// tests, and the coil sums run in coil order: the same bits.  1 572 864
-// samples, 12 coils: k_interp_grad 7.93 -> 3.31 ms, 2.4 ms with seven blocks
-// per SM (six and eight, which spills 1.4 KB: 2.5 and 2.8); its multiply-adds
-// and the weights formed anew per quad bound it now.  262 144 samples in four
-// bins, 8 coils: k_pair_grad 0.36 -> 0.11 ms a launch.
+// tests, and the coil sums run in coil order: the same bits.
+//
+// Bound by latency: registers decide how many warps hide it.  The 30 factors of
+// a sample in every lane's registers, with the 125 taps unrolled, spilled 390
+// bytes at seven blocks per SM; the x and y factors are now read from shared
+// memory where they are used, eight taps' loads in flight at a time.  1 572 864
+// samples, 12 coils: k_interp_grad 7.93 ms, this kernel with the factors in
+// registers 2.36 ms, now 1.14 ms at eight blocks per SM.  Sixteen loads in flight
+// at six blocks per SM cost 2 % of a loss evaluation more, four at eight 4 %,
+// six or seven blocks with eight loads 5 and 1 %, the rows unrolled 13 %.
 // ---------------------------------------------------------------------------
 struct GradSums {
     float2 y, d0, d1, d2;
 };
 
-// A sample's factors and their derivatives.  Where all three supports of every
-// sample of the warp hold exactly four candidates, these are moved to the
-// positions 0 .. 3 of each axis (`four`), else candidates sit at 0 .. 4.
+constexpr int QG_SAMPLES = 32;   // samples per block of 128 threads
+// shared floats of a sample: (factor, derivative) pairs of x, then of y; eight
+// samples this far apart fall in different banks
+constexpr int QG_PITCH = 20;
+
+// A sample's factors and their derivatives: along z in registers, along x and
+// y in shared memory, which the sample's four lanes share.  Where all three
+// supports of every sample of the warp hold exactly four candidates, these are
+// moved to the positions 0 .. 3 of each axis (`four`), else candidates sit at
+// 0 .. 4.
 struct QuadTaps {
-    float w[15], dw[15];
+    float wz[5], dwz[5];
+    const float* xy;
     long long base;   // grid point of candidate (0, 0, 0); may lie outside the grid unless four
     bool four;
 };
 
-// all 32 lanes of the warp
-CGS_D void quad_taps(const TapRecord* rec, const TapRecord* drec, long long i, int Gy, int Gz, QuadTaps& t)
+// all 32 lanes of the warp; xy: the sample's shared floats
+CGS_D void quad_taps(const TapRecord* rec, const TapRecord* drec, long long i, int Gy, int Gz, float* xy, QuadTaps& t)
 {
+    float w[15], dw[15];
     int nx, ny, nz, t0, t1, t2;
-    load_record(rec, i, t.w, nx, ny, nz);
-    load_record(drec, i, t.dw, t0, t1, t2);
+    load_record(rec, i, w, nx, ny, nz);
+    load_record(drec, i, dw, t0, t1, t2);
     bool ok = true;
     int sh[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const float* w = t.w + 5 * a;
-        sh[a] = w[0] == 0.f;
-        ok = ok && w[1] != 0.f && w[2] != 0.f && w[3] != 0.f && ((w[0] == 0.f) != (w[4] == 0.f));
+        const float* u = w + 5 * a;
+        sh[a] = u[0] == 0.f;
+        ok = ok && u[1] != 0.f && u[2] != 0.f && u[3] != 0.f && ((u[0] == 0.f) != (u[4] == 0.f));
     }
     t.four = __all_sync(0xffffffffu, ok);
     if (t.four) {
@@ -207,22 +222,34 @@ CGS_D void quad_taps(const TapRecord* rec, const TapRecord* drec, long long i, i
         for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                t.w[5 * a + q] = sh[a] ? t.w[5 * a + q + 1] : t.w[5 * a + q];
-                t.dw[5 * a + q] = sh[a] ? t.dw[5 * a + q + 1] : t.dw[5 * a + q];
+                w[5 * a + q] = sh[a] ? w[5 * a + q + 1] : w[5 * a + q];
+                dw[5 * a + q] = sh[a] ? dw[5 * a + q + 1] : dw[5 * a + q];
             }
         nx += sh[0];
         ny += sh[1];
         nz += sh[2];
     }
     t.base = ((long long)(nx - 2) * Gy + (ny - 2)) * Gz + (nz - 2);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        t.wz[q] = w[10 + q];
+        t.dwz[q] = dw[10 + q];
+    }
+    if ((threadIdx.x & 3) == 0) {
+#pragma unroll
+        for (int q = 0; q < 10; ++q) *reinterpret_cast<float2*>(xy + 2 * q) = make_float2(w[q], dw[q]);
+    }
+    __syncwarp();
+    t.xy = xy;
 }
 
-// The compiler must not keep the 125 taps' weights across the coils (it would
-// spill them): each coil's sums form them anew from the 30 factors.
-CGS_D void opaque(QuadTaps& t)
+// (factor, derivative): read where it is used (volatile), so that the compiler
+// does not keep the factors or the taps' weights across the coils
+CGS_D float2 xy_pair(const QuadTaps& t, int q)
 {
-#pragma unroll
-    for (int q = 0; q < 15; ++q) asm volatile("" : "+f"(t.w[q]), "+f"(t.dw[q]));
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_addr(t.xy + 2 * q)));
+    return v;
 }
 
 // Value and coordinate derivatives of one coil at one sample; g: the coil's
@@ -233,27 +260,28 @@ CGS_D GradSums quad_grad_run(const float2* __restrict__ g, const QuadTaps& t, in
     GradSums r;
     r.y = r.d0 = r.d1 = r.d2 = make_float2(0.f, 0.f);
     const float2* b = g + t.base * 4;
-#pragma unroll
-    for (int jx = 0; jx < N; ++jx)
-#pragma unroll
-        for (int y0 = 0; y0 < N; y0 += N == 4 ? 4 : 1) {
-            constexpr int NY = N == 4 ? 4 : 1;
+#pragma unroll 1   // unrolled, the compiler keeps the planes' addresses across the coils and spills
+    for (int jx = 0; jx < N; ++jx, b += (long long)Gy * Gz * 4) {
+        const float2 fx = xy_pair(t, jx);
+#pragma unroll 1
+        for (int y0 = 0; y0 < N; y0 += N == 4 ? 2 : 1) {
+            constexpr int NY = N == 4 ? 2 : 1;
             float2 v[NY][N];
 #pragma unroll
             for (int q = 0; q < NY; ++q) {
-                const float2* row = b + (long long)(jx * Gy + y0 + q) * Gz * 4;
-                const float wxy = t.w[jx] * t.w[5 + y0 + q];
+                const float2* row = b + (long long)(y0 + q) * Gz * 4;
+                const float wxy = N == 4 ? 0.f : fx.x * xy_pair(t, 5 + y0 + q).x;
 #pragma unroll
                 for (int jz = 0; jz < N; ++jz)   // with N = 4 every candidate lies in the grid
-                    if (N == 4 || wxy * t.w[10 + jz] > thresh) v[q][jz] = __ldg(row + jz * 4);
+                    if (N == 4 || wxy * t.wz[jz] > thresh) v[q][jz] = __ldg(row + jz * 4);
             }
 #pragma unroll
             for (int q = 0; q < NY; ++q) {
-                const float wx = t.w[jx], dwx = t.dw[jx], wy = t.w[5 + y0 + q], dwy = t.dw[5 + y0 + q];
-                const float wxy = wx * wy, ax = dwx * wy, ay = wx * dwy;
+                const float2 fy = xy_pair(t, 5 + y0 + q);
+                const float wxy = fx.x * fy.x, ax = fx.y * fy.x, ay = fx.x * fy.y;
 #pragma unroll
                 for (int jz = 0; jz < N; ++jz) {
-                    const float wz = t.w[10 + jz], dwz = t.dw[10 + jz];
+                    const float wz = t.wz[jz], dwz = t.dwz[jz];
                     const float wt = wxy * wz;   // 0 outside the support or the grid
                     if (wt > thresh) {
                         const float ex = ax * wz, ey = ay * wz, ez = wxy * dwz;
@@ -269,6 +297,7 @@ CGS_D GradSums quad_grad_run(const float2* __restrict__ g, const QuadTaps& t, in
                 }
             }
         }
+    }
     return r;
 }
 CGS_D GradSums quad_grad_sums(const float2* __restrict__ g, const QuadTaps& t, int Gy, int Gz, float thresh)
@@ -276,11 +305,10 @@ CGS_D GradSums quad_grad_sums(const float2* __restrict__ g, const QuadTaps& t, i
     return t.four ? quad_grad_run<4>(g, t, Gy, Gz, thresh) : quad_grad_run<5>(g, t, Gy, Gz, thresh);
 }
 
-constexpr int QG_SAMPLES = 32;   // samples per block of 128 threads
-
-__global__ void __launch_bounds__(4 * QG_SAMPLES, 7) k_interp_grad_quad(InterpGradArgs a)
+__global__ void __launch_bounds__(4 * QG_SAMPLES, 8) k_interp_grad_quad(InterpGradArgs a)
 {
     __shared__ double s_red[QG_SAMPLES / 8];
+    __shared__ __align__(8) float s_xy[QG_SAMPLES * QG_PITCH];
     const int lane = threadIdx.x & 31, sub = threadIdx.x & 3, lead = lane & ~3;
     const long long j = (long long)blockIdx.x * QG_SAMPLES + threadIdx.x / 4;
     const bool on = j < a.n;
@@ -289,11 +317,10 @@ __global__ void __launch_bounds__(4 * QG_SAMPLES, 7) k_interp_grad_quad(InterpGr
     const long long i = a.s0 + (on ? j : 0);
     if (a.n > 0) {
         QuadTaps t;
-        quad_taps(a.rec, a.drec, i, a.G[1], a.G[2], t);
+        quad_taps(a.rec, a.drec, i, a.G[1], a.G[2], s_xy + QG_PITCH * (threadIdx.x / 4), t);
         const float D = a.dcf ? a.dcf[i] : 1.f;
         for (int c0 = 0; c0 < a.nch; c0 += 4) {
             const int c = c0 + sub;
-            opaque(t);
             const GradSums r = quad_grad_sums(a.grid + (long long)(c0 / 4) * a.coil_stride + sub, t, a.G[1], a.G[2],
                                               a.thresh);
             float p0 = 0.f, p1 = 0.f, p2 = 0.f;
@@ -467,19 +494,19 @@ __global__ void __launch_bounds__(128) k_pair_grad(PairGradArgs a)
     }
 }
 
-__global__ void __launch_bounds__(4 * QG_SAMPLES, 6) k_pair_grad_quad(PairGradArgs a)
+__global__ void __launch_bounds__(4 * QG_SAMPLES, 8) k_pair_grad_quad(PairGradArgs a)
 {
+    __shared__ __align__(8) float s_xy[QG_SAMPLES * QG_PITCH];
     const int lane = threadIdx.x & 31, sub = threadIdx.x & 3, lead = lane & ~3;
     const long long j = (long long)blockIdx.x * QG_SAMPLES + threadIdx.x / 4;
     const bool on = j < a.n;
     const long long i = a.s0 + (on ? j : 0);
     QuadTaps t;
-    quad_taps(a.rec, a.drec, i, a.G[1], a.G[2], t);
+    quad_taps(a.rec, a.drec, i, a.G[1], a.G[2], s_xy + QG_PITCH * (threadIdx.x / 4), t);
     const float D = a.dcf ? a.dcf[i] : 1.f;
     float gk[3] = {0.f, 0.f, 0.f};
     for (int c0 = 0; c0 < a.nch; c0 += 4) {
         const int c = c0 + sub;
-        opaque(t);
         const GradSums r = quad_grad_sums(a.grid + (long long)(c0 / 4) * a.coil_stride + sub, t, a.G[1], a.G[2],
                                           a.thresh);
         const long long e = i * a.nch + c;

@@ -74,3 +74,42 @@ def test_sliced_gather_equals_tiled_kernel_bitwise(gpu_lib, cgs, img, grid, nch,
     r.set_launch_shape(0, 1, 2)
     x1, res1, _ = r.cg_sense_batched(y, 0.0, 3)
     assert np.array_equal(x6, x1) and np.array_equal(res6, res1)
+
+
+@pytest.mark.parametrize("nch,coil", [(3, 2), (4, 1), (5, 4), (9, 6)])
+@pytest.mark.parametrize("kb_w", [4.0, 4.25])
+@pytest.mark.parametrize("ns", [1, 33, 800])
+def test_quad_loss_gradients_equal_coil_planes(gpu_lib, cgs, nch, coil, kb_w, ns):
+    """Loss, dL/dk and dL/dx with one coil's map and data non-zero against a
+    single-coil reconstruction (coil planes): warps whose samples all hold four
+    candidates an axis and others, at the grid's faces, part-filled warps and
+    blocks.  The residual and the derivative sums are the same bits; the loss
+    adds them in FP64 in another order (1e-12) and dL/dk rounds two products and
+    their sum per coil (a few 6e-8: 1e-6)."""
+    import torch
+    rng = np.random.default_rng(8)
+    img, grid = (16, 16, 12), (32, 32, 24)
+    k = rng.uniform(0, 1, (ns, 3))
+    k[:6] = np.array([[0, 0, 0], [1, 1, 1], [0, 1, 0.5], [1, 0, 0.5], [0.5, 0, 1], [0.5, 1, 0]])[:min(ns, 6)]
+    one = (rng.standard_normal(img) + 1j * rng.standard_normal(img)).astype(np.complex64)
+    maps = np.zeros((nch,) + img, np.complex64)
+    maps[coil] = one
+    y = np.zeros((nch, ns), np.complex64)
+    y[coil] = rng.standard_normal(ns) + 1j * rng.standard_normal(ns)
+    x = torch.from_numpy((rng.standard_normal(img) + 1j * rng.standard_normal(img)).astype(np.complex64)).cuda()
+    dcf = rng.uniform(0.5, 1.5, ns).astype(np.float32)
+    got = []
+    for n, m, d in ((nch, maps, y), (1, maps[coil:coil + 1], y[coil:coil + 1])):
+        r = cgs.Reco(img, grid, n, kb_w=kb_w, kb_b=9.0)
+        r.set_trajectory(k)
+        r.set_dcf(dcf)
+        r.set_smaps(m)
+        gx = torch.zeros_like(x)
+        gk = torch.zeros((ns, 3), dtype=torch.float32, device="cuda")
+        loss = r.loss_grad_tensor(x, torch.from_numpy(np.ascontiguousarray(d)).cuda(), gx, gk)
+        got.append((loss, gx.cpu().numpy(), gk.cpu().numpy()))
+    (la, xa, ka), (lb, xb, kb) = got
+    assert lb > 0 and np.abs(kb).max() > 0
+    assert abs(la - lb) < 1e-12 * lb
+    assert np.array_equal(xa, xb)
+    assert np.linalg.norm(ka - kb) < 1e-6 * np.linalg.norm(kb)
