@@ -72,6 +72,18 @@ FAMILY = {"fwd_z": "k_fwd_z_pipe+k_adj_z_pipe", "adj_z": "k_fwd_z_pipe+k_adj_z_p
           "spread_adjx": "k_spread_adjx"}
 
 
+def families(n_ch, variant, gather):
+    """FAMILY for a coil count and spreading variant: from three coils on the
+    forward grid lies in quads of coils, and variant 6 (the transposed matrix
+    in slices) spreads into the same layout."""
+    f = dict(FAMILY, spread="k_spread_csr" if gather else "k_spread")
+    if n_ch >= 3:
+        f.update(fwd_x="k_fwd_x_quad", interp="k_interp_quad")
+        if gather and variant == 6:
+            f.update(spread="k_spread_quad", adj_x="k_adj_x_quad")
+    return f
+
+
 def traffic_record():
     """DRAM bytes (read + write) against algorithmic bytes of each kernel
     family in one application of the first two cfg3 bins, from an ncu capture
@@ -288,7 +300,34 @@ def make_workload(cgs, synth, torch, name, device, stream_handle, dcf_kind="voro
     return w, reco, data, sbins, smaps, dcf, k, kb_w, kb_b, dcf_s
 
 
-def stage_bytes(w, sizes, support=None, matrix=None, y_listed=False, fused=False):
+def touched_points(w, k, bins, kb_w):
+    """Grid points that some sample's kernel support covers, summed over the
+    bins (at 12 coils three 32-byte sectors each: what the passes over quads of
+    coils store and load)."""
+    import torch
+    dev = torch.device("cuda")
+    total = 0
+    off = torch.arange(-2, 3, device=dev)
+    for idx in bins:
+        mark = torch.zeros(int(np.prod(w.grid)), dtype=torch.bool, device=dev)
+        for i0 in range(0, len(idx), 1 << 16):
+            kk = torch.from_numpy(np.ascontiguousarray(k[np.asarray(idx[i0:i0 + (1 << 16)])], np.float64)).to(dev)
+            lin, ok = None, None
+            for a in range(3):
+                u = kk[:, a] * w.grid[a]
+                j = torch.round(u).long()[:, None] + off
+                on = ((j - u[:, None]).abs() <= kb_w / 2) & (j >= 0) & (j < w.grid[a])
+                shape = [len(kk), 1, 1, 1]
+                shape[a + 1] = 5
+                j, on = j.reshape(shape), on.reshape(shape)
+                lin = j if lin is None else lin * w.grid[a] + j
+                ok = on if ok is None else ok & on
+            mark[lin[ok]] = True
+        total += int(mark.sum())
+    return total
+
+
+def stage_bytes(w, sizes, support=None, matrix=None, y_listed=False, fused=False, touched=0, slices=False):
     """Algorithmic bytes of each stage of one E^H D E application over all
     bins: every stage reads its input and writes its output once.
     support = (listed columns, stored spreading tiles) per bin, from
@@ -302,7 +341,10 @@ def stage_bytes(w, sizes, support=None, matrix=None, y_listed=False, fused=False
     listed columns' rows (8 bytes x Ix per listed column).  fused: the
     gather runs fused with the adjoint x pass (stage "spread_adjx"): the
     matrix and the samples are read, the x pass's Ix output rows written,
-    the grid never stored or reloaded."""
+    the grid never stored or reloaded.  touched (touched_points): the grid
+    lies in quads of coils, of which the forward x pass stores and the
+    interpolation loads these points only; slices: so do the spreading, which
+    then reads the taps without row offsets, and the adjoint x pass."""
     Ix, Iy, Iz = w.img
     Gx, Gy, Gz = w.grid
     Ni, Ng, Nl = Ix * Iy * Iz, Gx * Gy * Gz, Ix * Iy
@@ -316,10 +358,11 @@ def stage_bytes(w, sizes, support=None, matrix=None, y_listed=False, fused=False
         cols, tiles = [int(v) for v in support[0]], [int(v) for v in support[1]]
     scol, stile = sum(cols), sum(tiles)
     if fused and matrix:
-        sb = stage_bytes(w, sizes, support, matrix, y_listed)
+        sb = stage_bytes(w, sizes, support, matrix, y_listed, touched=touched)
         sb["spread_adjx"] = 4 * matrix[1] + 8 * matrix[0] + M * C8 + C8 * scol * Ix
         return {k: sb[k] for k in STAGES_FUSED}
-    return {
+    quads = 32 * ((w.n_ch + 3) // 4) * touched
+    sb = {
         # the coil maps once per application: the z passes run the bins of a
         # line block side by side, so the other bins read the maps from L2
         "fwd_z": nb * (8 * Ni + C8 * Nl * Gz) + C8 * Ni,
@@ -332,13 +375,20 @@ def stage_bytes(w, sizes, support=None, matrix=None, y_listed=False, fused=False
         "adj_y": nb * C8 * (Ix * Gy * Gz + Nl * Gz),
         "adj_z": nb * (C8 * Nl * Gz + 8 * Ni) + C8 * Ni,
     }
+    if touched:
+        sb["fwd_x"] = C8 * scol * Ix + quads
+        sb["interp"] = quads + M * (64 + 4 + C8)
+        if slices:
+            sb["spread"] = quads + 8 * matrix[0] + M * C8
+            sb["adj_x"] = quads + C8 * scol * Ix
+    return sb
 
 
-def apply_bytes(w, sizes, support=None, matrix=None, y_listed=False, fused=False):
+def apply_bytes(w, sizes, support=None, matrix=None, y_listed=False, fused=False, touched=0, slices=False):
     """Algorithmic bytes of one application of the operator (its eight
     stages, seven fused; the CG vector updates of a solve, 64 bytes per voxel
     and bin and iteration, are not part of it)."""
-    return sum(stage_bytes(w, sizes, support, matrix, y_listed, fused).values())
+    return sum(stage_bytes(w, sizes, support, matrix, y_listed, fused, touched, slices).values())
 
 
 # ---------------------------------------------------------------------------
@@ -992,9 +1042,12 @@ def run_ours(args):
         support = reco.support_stats()
         taps, points = reco.spread_matrix_stats()
         fused = reco.spread_fused()
+        touched = touched_points(w, k, sbins, kb_w) if w.n_ch >= 3 else 0
+        slices = bool(touched) and taps > 0 and args.spread_variant in (0, 6) and not fused
         print(json.dumps({"applies": args.applies_only, "bins": nb, "spread_fused_with_adjoint_x": fused,
+                          "touched_points": touched,
                           "algorithmic_bytes": stage_bytes(w, sizes, support, (taps, points) if taps > 0 else None,
-                                                           reco.forward_y_listed_rows(), fused)}))
+                                                           reco.forward_y_listed_rows(), fused, touched, slices)}))
         return 0
 
     t0 = time.perf_counter()
@@ -1176,14 +1229,17 @@ def run_ours(args):
     del b_rhs
     support = reco.support_stats()
     taps, points = reco.spread_matrix_stats()
-    variant = tune.get("spread_variant") if tune else 8   # the library's default is the fused gather
+    variant = tune.get("spread_variant") if tune else 8 if fused else 6   # untuned: the library's rule
     gather = variant in (6, 7, 8) and taps > 0
     matrix = (taps, points) if gather else None
     y_listed = reco.forward_y_listed_rows()
-    sb = stage_bytes(w, sizes, support, matrix, y_listed, fused)
+    touched = touched_points(w, k, sbins, kb_w) if w.n_ch >= 3 else 0
+    slices = bool(touched) and gather and variant == 6
+    form = (w, sizes, support, matrix, y_listed, fused, touched, slices)
+    sb = stage_bytes(*form)
     apply_ms = float(sum(stage_ms.values()))
     # kernel families: the x/y passes are one kernel template
-    family = dict(FAMILY, spread="k_spread_csr" if gather else "k_spread")
+    family = families(w.n_ch, variant, gather)
     fam = {k: [s for s in names if family[s] == k] for k in dict.fromkeys(family[s] for s in names)}
     fam_ms = {k: sum(stage_ms[s] for s in v) for k, v in fam.items()}
     dom = max(fam_ms, key=fam_ms.get)
@@ -1210,8 +1266,8 @@ def run_ours(args):
         "apply_ms": apply_ms,
         "rhs_ms": rhs_ms,
         "cg_update_ms_per_iter": (ms_step - iters * apply_ms - rhs_ms) / max(iters, 1),
-        "apply_achieved_gbs": apply_bytes(w, sizes, support, matrix, y_listed, fused) / (apply_ms / 1e3) / 1e9,
-        "apply_bytes": apply_bytes(w, sizes, support, matrix, y_listed, fused),
+        "apply_achieved_gbs": apply_bytes(*form) / (apply_ms / 1e3) / 1e9,
+        "apply_bytes": apply_bytes(*form),
         "spread_fused_with_adjoint_x": fused,
         "support": {"listed_column_fraction": float(sum(support[0])) / (nb * w.grid[1] * w.grid[2]),
                     "stored_tile_fraction": float(sum(support[1])) / (nb * int(np.prod(w.grid)) // 512)},
