@@ -609,7 +609,8 @@ cudaError_t launch_pm_init(float* w, float2* v, long long n, cudaStream_t s)
 // update.  Sums run in the order of k_spread and k_interp with the same fused
 // multiply-adds: the same weights bit for bit.  16 bins, 1 572 864 samples,
 // grid 256 x 256 x 192, an iteration: k_spread 1.46 + k_interp 0.18 ms against
-// 0.66 + 0.20 (the rows' scattered reads bound the gather).
+// 0.66 + 0.20 (the rows' scattered reads bound the gather); over slices, where
+// the matrix is in that form (k_pm_slices), 0.31 + 0.20.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_pm_spread(PmArgs a)
 {

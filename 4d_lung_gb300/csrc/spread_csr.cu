@@ -803,7 +803,9 @@ cudaError_t launch_spread_quad(const SliceSpreadArgs& a, bool kahan, cudaStream_
     return cudaGetLastError();
 }
 
-// The real gather of the density weights: the same slices
+// The real gather of the density weights: the same slices, one lane a point.
+// Bound by the sectors of its 4-byte reads: 1.57 M samples in 16 bins 0.66 ms by
+// rows, 0.31 ms here; entries fetched ahead of their use 2-4 % slower.
 __global__ void __launch_bounds__(32 * SQ_WARPS) k_pm_slices(SliceSpreadArgs a)
 {
     const long long J = a.j0 + blockIdx.x;
