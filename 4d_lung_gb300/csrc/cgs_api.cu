@@ -7,6 +7,7 @@
 #include "cgsense_c.h"
 #include "launch.h"
 #include "fft_sizes.h"
+#include "kb_series.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -261,40 +262,6 @@ double kb_factor(const cgs_params& p, int n, double dist)
     const float q = (float)(2.f * d) / (float)(w * dk);
     const double arg = (double)b * std::sqrt(1.0 - (double)q * (double)q);
     return std::cyl_bessel_i(0.0, arg) / (double)(float)(100.0f * w * dk);
-}
-
-float2 float_pair(double v)
-{
-    const float h = (float)v;
-    return make_float2(h, (float)(v - (double)h));
-}
-
-// I0(b sqrt(s)) (order 0) or I1(b sqrt(s)) / sqrt(s) (order 1) as a power
-// series in s (Abramowitz and Stegun 9.6.10): c_k = (b/2)^order (b^2/4)^k /
-// (k! (k + order)!), all positive.  Terms until their sum at s = 1 no longer
-// changes; the tail that makes up less than 2^-30 of it goes to FP32 (its share
-// is largest at s = 1).  nd = 0 when the shape needs more than the arrays hold.
-KbSeries kb_series_of(double b, int order)
-{
-    std::vector<double> c;
-    double t = order ? 0.5 * b : 1.0, sum = 0.0;
-    for (int k = 0; k < 200; ++k) {
-        c.push_back(t);
-        sum += t;
-        t *= 0.25 * b * b / ((double)(k + 1) * (double)(k + 1 + order));
-        if (t < 1e-18 * sum && 0.25 * b * b < (double)(k + 1) * (double)(k + 1)) break;
-    }
-    int nd = (int)c.size();
-    double tail = 0.0;
-    while (nd > 1 && tail + c[nd - 1] < sum * 0x1p-30) tail += c[--nd];
-    KbSeries s{};
-    const int nf = (int)c.size() - nd;
-    if (!(b >= 0.0) || !std::isfinite(sum) || nd > KB_ND || nf > KB_NF) return s;
-    s.nd = nd;
-    s.nf = nf;
-    for (int k = 0; k < nd; ++k) s.cd[k] = float_pair(c[k]);
-    for (int k = 0; k < nf; ++k) s.cf[k] = (float)c[nd + k];
-    return s;
 }
 
 // ConvKernel::calculateKernelFT (Reco.cpp:560-601) is separable: the 3-D
@@ -645,12 +612,7 @@ KbParams kb_params(const cgs_ctx* c)
     kb.thresh = c->thresh;
     kb.i0 = c->kb_i0;
     kb.i1 = c->kb_i1;
-    for (int a = 0; a < 3; ++a) {
-        const float dk = (float)(1.0 / (double)(float)(c->G[a] - 1));
-        const double C = (double)(float)(100.0f * kb.w * dk);
-        kb.rC[a] = float_pair(1.0 / C);
-        kb.f0[a] = float_pair((double)kb.b * (2.0 / ((double)kb.w * (double)dk)) / C);
-    }
+    kb_scales(kb);
     return kb;
 }
 

@@ -50,11 +50,14 @@ __global__ void k_tap_grad_records(const double* __restrict__ k, const int* __re
                 const float d = (float)fabs(dd);
                 if (!(d > wHalf * dk)) {
                     const float q = (float)(2.f * d) / (float)(kb.w * dk);
-                    float dv;
-                    if (kb.i1.nd > 0) {
-                        const float2 f = pair_mul(make_float2(q, 0.f), kb.f0[a]);
-                        dv = -pair_mul(kb_series(kb.i1, pair_one_minus_sq(q)), f).x;
-                    } else {
+                    float dv = 0.f;
+                    bool sure = kb.i1.nd > 0;
+                    if (sure) {
+                        const float2 p = kb_slope(kb, a, q);
+                        dv = -p.x;
+                        sure = pair_rounds(p);
+                    }
+                    if (!sure) {
                         const double s2 = __dadd_rn(1.0, -__dmul_rn((double)q, (double)q));
                         const double s = s2 > 0.0 ? sqrt(s2) : 0.0;
                         const double b = (double)kb.b;

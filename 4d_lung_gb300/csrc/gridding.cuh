@@ -29,9 +29,10 @@ namespace cgs {
 // float product (index * float dk), then a float distance.  The Bessel factor
 // I0(b sqrt(1 - q^2)) is its power series in 1 - q^2 on float pairs (kb_series):
 // bound by the FP64 pipe, the library function with its square root and
-// division cost 54 FP64 operations a candidate; now there are 3.  262 144
-// samples: 336 us, 217 with the series in FP64, 67 with float pairs (the
-// derivative records 472, 255, 74).
+// division cost 54 FP64 operations a candidate; now there are 3, but for the one
+// candidate in some 10^5 whose float the pair cannot decide (pair_rounds): the
+// records hold the FP64 form's floats.  262 144 samples: 336 us, 217 with the
+// series in FP64, 67 with float pairs (the derivative records 472, 255, 74).
 // ---------------------------------------------------------------------------
 __global__ void k_tap_records(const double* __restrict__ k, const int* __restrict__ sample_idx,
                               long long n, KbParams kb, TapRecord* __restrict__ out)
@@ -57,9 +58,13 @@ __global__ void k_tap_records(const double* __restrict__ k, const int* __restric
                 const float d = (float)fabs(dd);
                 if (!(d > wHalf * dk)) {
                     const float q = (float)(2.f * d) / (float)(kb.w * dk);
-                    if (kb.i0.nd > 0) {
-                        val = pair_mul(kb_series(kb.i0, pair_one_minus_sq(q)), kb.rC[a]).x;
-                    } else {
+                    bool sure = kb.i0.nd > 0;
+                    if (sure) {
+                        const float2 p = kb_value(kb, a, q);
+                        val = p.x;
+                        sure = pair_rounds(p);
+                    }
+                    if (!sure) {
                         const double arg = (double)kb.b * sqrt(__dadd_rn(1.0, -__dmul_rn((double)q, (double)q)));
                         val = (float)(cyl_bessel_i0(arg) / (double)(float)(100.0f * kb.w * dk));
                     }
