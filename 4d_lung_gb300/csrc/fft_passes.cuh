@@ -1067,8 +1067,10 @@ k_fwd_z_pipe(FwdZArgs a)
     const bool act2 = ln2 < LPB && line2 < a.nl;
 
     // the thread's twiddles, the same for every coil, where the registers allow
-    // (lines of 192 measured 5 % slower with them: spills at 4 blocks per SM)
-    constexpr bool TWR = R1 > 16 || R2 > 16;
+    // (lines of 192 measured 5 % slower with them: spills at 4 blocks per SM; the
+    // 32 twiddles of a line of 352 beside its 32 values spill too: 20 coils of
+    // 256 x 256 lines 1.31 -> 1.45 ms)
+    constexpr bool TWR = R2 > 16 && R1 <= 16;
     float2 twr[TWR ? R1 : 1];
     if constexpr (TWR) {
 #pragma unroll
@@ -1186,9 +1188,14 @@ k_adj_z_pipe(AdjZArgs a)
 #pragma unroll
     for (int j = 0; j < K1 - K0; ++j) acc[j] = make_float2(0.f, 0.f);
 
-    float2 twr[R1];   // the thread's twiddles, the same for every coil
+    // the thread's twiddles, the same for every coil, where the registers allow
+    // (the 32 of a line of 352 would halve the resident warps: 1.21 -> 1.48 ms)
+    constexpr bool TWR = R1 <= 16;
+    float2 twr[TWR ? R1 : 1];
+    if constexpr (TWR) {
 #pragma unroll
-    for (int kk = 1; kk < R1; ++kk) twr[kk] = s_tw[n2 * (R1 + 1) + kk];
+        for (int kk = 1; kk < R1; ++kk) twr[kk] = s_tw[n2 * (R1 + 1) + kk];
+    }
     for (int c = 0; c < a.nch; ++c) {
         const int st = c % NST;
         const bool ok = mbar_wait_bounded(&s_bar[st], (uint32_t)((c / NST) & 1), PIPE_WAIT_NS);
@@ -1216,7 +1223,7 @@ k_adj_z_pipe(AdjZArgs a)
 #pragma unroll
             for (int kk = 0; kk < R1; ++kk) {
                 float2 t = v[kk];
-                if (kk > 0) t = table_twiddle<SIGN>(t, twr[kk]);
+                if (kk > 0) t = table_twiddle<SIGN>(t, TWR ? twr[TWR ? kk : 0] : s_tw[n2 * (R1 + 1) + kk]);
                 else if (INF) t = parity(t, n2);
                 s_y[ln1 * Lay::LINE + n2 * Lay::R1P + kk] = t;
             }
