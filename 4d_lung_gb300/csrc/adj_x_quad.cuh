@@ -24,8 +24,10 @@ struct AdjQuadLayout {
     static constexpr int NT = Q::NT;
     // blocks of 256 threads, four per SM (64 registers): their loads and
     // transforms overlap better than two blocks of 8 columns (16 bins of the
-    // 256 x 256 x 192 grid, 12 coils: 2.43 -> 2.32 ms; three blocks 2.47)
-    static constexpr int MINB = Q::RM <= 16 ? 4 : Q::MINB;
+    // 256 x 256 x 192 grid, 12 coils: 2.43 -> 2.32 ms; three blocks 2.47).  Lines
+    // of 352, 448 and 512 points: 8 columns (fft_adj_quad_tile_cols), 512 threads
+    // of 128 registers, the stage of more than 16 rows in two turns.
+    static constexpr int MINB = Q::RM <= 16 ? 4 : Q::NT > 384 ? 1 : Q::MINB;
     static constexpr size_t smem_bytes = ((size_t)Q::L * Q::W + Q::L + R2) * sizeof(float2);
 };
 
@@ -53,9 +55,7 @@ k_adj_x_quad(AdjXQuadArgs a, int nunits, int per_quad, int nsub)
     __syncthreads();
     const int nq = (a.nch + 3) / 4;
     // stage 1: coil fastest, then column, then n2; stage 2: column fastest, then k1, then coil
-    const int coil1 = tid & 3, col1 = (tid >> 2) % TBQ, n2 = tid / W;
-    const int col2 = tid % TBQ, g2 = tid / TBQ;
-    const int coil2 = g2 / R1, k1s = g2 - coil2 * R1;
+    const int coil1 = tid & 3, col1 = (tid >> 2) % TBQ, col2 = tid % TBQ;
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const int q = u / per_quad, rem = u - q * per_quad;   // quads outer, as the forward pass
         const int t = rem / nsub, s = rem - t * nsub;
@@ -63,8 +63,7 @@ k_adj_x_quad(AdjXQuadArgs a, int nunits, int per_quad, int nsub)
         const int nc = min(4, a.nch - 4 * q);
         const long long slot = e.x - a.bin0;
         const int b0 = e.y + s * TBQ;
-        float2 v[R1];
-        if (n2 < R2) {
+        auto rows = [&](float2 (&v)[R1], int n2) {
 #pragma unroll
             for (int n1 = 0; n1 < R1; ++n1) v[n1] = make_float2(0.f, 0.f);
             if (coil1 < nc) {
@@ -87,15 +86,30 @@ k_adj_x_quad(AdjXQuadArgs a, int nunits, int per_quad, int nsub)
                 else if (k1 > 0) tv = table_twiddle<SIGN>(tv, s_tw[n2 * k1]);
                 v[k1] = tv;
             }
-        }
-        // the exchange is free once every thread has left stage 2 of the last unit
-        __syncthreads();
-        if (n2 < R2) {
+        };
+        auto put = [&](const float2 (&v)[R1], int n2) {
 #pragma unroll
             for (int k1 = 0; k1 < R1; ++k1) s_y[(k1 * R2 + n2) * W + Q::slot(coil1, col1, k1)] = v[k1];
+        };
+        const int n2 = tid / W;
+        float2 v[R1];
+        if (n2 < R2) rows(v, n2);
+        // the exchange is free once every thread has left stage 2 of the last unit
+        __syncthreads();
+        if (n2 < R2) put(v, n2);
+#pragma unroll 1
+        for (int turn = 1; turn < Q::T1; ++turn) {
+            const int m2 = n2 + turn * Q::NG;
+            if (m2 >= R2) break;
+            rows(v, m2);
+            put(v, m2);
         }
         __syncthreads();
-        if (coil2 < nc) {
+#pragma unroll 1
+        for (int turn = 0; turn < Q::T2; ++turn) {
+            const int g2 = tid / TBQ + turn * (NT / TBQ);
+            const int coil2 = g2 / R1, k1s = g2 - coil2 * R1;
+            if (coil2 >= nc) break;
             float2 w[R2];
 #pragma unroll
             for (int m = 0; m < R2; ++m) w[m] = s_y[(k1s * R2 + m) * W + Q::slot(coil2, col2, k1s)];

@@ -64,7 +64,7 @@ struct SizeImpl {
     static constexpr int NSTAGE_NI = 3;
     // forward x pass over quads of coils: unit widths of the two forms
     static constexpr int TBQ_IN = fft_quad_tile_cols(R1, R2, true), TBQ_NO = fft_quad_tile_cols(R1, R2, false);
-    static constexpr int TBQ_ADJ = 4;   // of the adjoint x pass from it
+    static constexpr int TBQ_ADJ = fft_adj_quad_tile_cols(R1, R2);   // of the adjoint x pass from it
 
     template <int SIGN, int MODE, int TBK = TB, int NS = NSTAGE>
     static cudaError_t tma_attr(int smem)

@@ -28,6 +28,13 @@ constexpr int fft_quad_tile_cols(int r1, int r2, bool half_in)
     return (r1 > r2 ? r1 : r2) > 16 || (!half_in && r1 * r2 >= 160) ? 4 : 8;
 }
 
+// columns of a unit of the adjoint x pass from the quad grid (adj_x_quad.cuh):
+// 8 (64-byte rows of the y buffer, one block of 512 threads per SM) where the
+// codelets have more than 24 points, else 4.  20 coils of a 512 x 512 x 352 grid:
+// 5.09 ms with 4 columns, 3.99 with 8 (4.10 -> 3.47 with few samples); 8 coils of
+// 448 and 512 x 192 x 192: 283 -> 288 and 295 -> 296 us.
+constexpr int fft_adj_quad_tile_cols(int r1, int r2) { return (r1 > r2 ? r1 : r2) > 24 ? 8 : 4; }
+
 // spreading fused with the adjoint x pass (spread_adjx.cuh): threads per
 // block, columns per tile (the x passes' narrow tiles)
 constexpr int SAX_NT = 1024, SAX_TB = 8;

@@ -22,7 +22,7 @@
 // in the grid); the exchange rows between them are XOR-swizzled so that both
 // sides are free of bank conflicts.  Units of 8 columns (512 threads, two
 // blocks per SM) where the input is half-pruned and the codelets have at most
-// 16 points, else 4 (the 32-point codelets' registers, twice the input rows).
+// 16 points, else 4 (the longer codelets' registers, twice the input rows).
 //
 // Measured, 16 bins of 128 x 128 x 96, 12 coils (grid 256 x 256 x 192), against
 // coil planes: this pass 2.83 -> 1.98 ms, the interpolation after it 3.19 ->
@@ -38,11 +38,21 @@ struct QuadLayout {
     static constexpr int L = R1 * R2;
     static constexpr int RM = R1 > R2 ? R1 : R2;
     static constexpr int W = 4 * TBQ;            // exchange row: coils x columns
-    static constexpr int NT = W * RM;
+    // thread groups of W: one per row group of the longer codelet's stage up to
+    // 24, else 16, and a stage with more rows takes them in two turns.  A 28- or
+    // 32-point codelet wants 128 registers: 16 W threads are two blocks per SM,
+    // all busy in its stage, where RM W threads were one, half idle there.  20
+    // coils of a 512 x 512 x 352 grid: 4.64 -> 3.33 ms (coil planes 3.98); 8
+    // coils of 352, 448 and 512 x 192 x 192: 404, 355, 349 -> 232, 227, 229 us
+    // (coil planes 301, 271, 286).  Images of more than 340 of 512 rows leave room
+    // for one block (417 rows: 397 -> 438 us, coil planes 1006).
+    static constexpr int NG = RM <= 24 ? RM : 16;
+    static constexpr int NT = W * NG;
+    static constexpr int T1 = (R2 + NG - 1) / NG, T2 = (R1 + NG - 1) / NG;   // turns of the two stages
     // resident blocks asked of the compiler: 64 to 102 registers a thread (two
     // of L = 320's blocks per SM instead of one: 1.31 -> 0.77 ms, 16 coils of
     // a 320 x 320 x 224 grid)
-    static constexpr int MINB = RM <= 16 ? (NT <= 256 ? 3 : 2) : RM <= 24 ? 2 : 1;
+    static constexpr int MINB = RM <= 16 ? (NT <= 256 ? 3 : 2) : 2;
     static constexpr int R2W = (R2 + 3) / 4;     // mask words of a row group k1
     // the x rows of one coil, rounded up to 128 bytes
     __host__ __device__ static int coil_elems(int rows) { return (rows * TBQ + 15) & ~15; }
@@ -119,29 +129,10 @@ k_fwd_x_quad(FwdXQuadArgs a, const __grid_constant__ CUtensorMap tmap, int nunit
     };
 
     // stage 1: column fastest, then n2, then coil; stage 2: coil fastest, then column, then k1
-    const int col1 = tid % TBQ, g1 = tid / TBQ;
-    const int coil1 = g1 / R2, n2 = g1 - coil1 * R2;
-    const bool act1 = coil1 < 4;
-    const int coil2 = tid & 3, col2 = (tid >> 2) % TBQ, k1 = tid / W;
-    const bool act2 = k1 < R1;
-    const int slot1 = Q::slot(coil1 & 3, col1, n2);
-
-    if (tid == 0 && my_n > 0) issue(0);
-    for (int k = 0; k < my_n; ++k) {
-        const bool ok = mbar_wait_bounded(s_bar, (uint32_t)(k & 1), PIPE_WAIT_NS);
-        if (__syncthreads_or(!ok)) {
-            // timeout: report, let the copies already issued land, leave
-            if (tid == 0) {
-                atomicExch(a.err, 1);
-                mbar_wait_bounded(s_bar, (uint32_t)(k & 1), PIPE_WAIT_NS);
-            }
-            return;
-        }
-        const int4 un = s_unit[k & 1];
-        // touch-mask bytes of this thread's row group k1 (one per k2, a bit per column)
-        uint32_t mw[Q::R2W];
+    const int col1 = tid % TBQ, coil2 = tid & 3, col2 = (tid >> 2) % TBQ;
+    auto load_mask = [&](uint32_t (&mw)[Q::R2W], int entry, int k1) {
         if (a.mask) {
-            const uint32_t* m = a.mask + ((long long)un.w * R1 + (act2 ? k1 : 0)) * Q::R2W;
+            const uint32_t* m = a.mask + ((long long)entry * R1 + k1) * Q::R2W;
             if constexpr (Q::R2W % 4 == 0) {
 #pragma unroll
                 for (int w = 0; w < Q::R2W / 4; ++w) {
@@ -159,7 +150,29 @@ k_fwd_x_quad(FwdXQuadArgs a, const __grid_constant__ CUtensorMap tmap, int nunit
 #pragma unroll
             for (int w = 0; w < Q::R2W; ++w) mw[w] = 0xffffffffu;
         }
-        if (act1) {
+    };
+
+    if (tid == 0 && my_n > 0) issue(0);
+    for (int k = 0; k < my_n; ++k) {
+        const bool ok = mbar_wait_bounded(s_bar, (uint32_t)(k & 1), PIPE_WAIT_NS);
+        if (__syncthreads_or(!ok)) {
+            // timeout: report, let the copies already issued land, leave
+            if (tid == 0) {
+                atomicExch(a.err, 1);
+                mbar_wait_bounded(s_bar, (uint32_t)(k & 1), PIPE_WAIT_NS);
+            }
+            return;
+        }
+        const int4 un = s_unit[k & 1];
+        // touch-mask bytes of a row group k1 (one per k2, a bit per column), of the first turn ahead
+        uint32_t mw[Q::R2W];
+        load_mask(mw, un.w, tid / W < R1 ? tid / W : 0);
+#pragma unroll 1
+        for (int turn = 0; turn < Q::T1; ++turn) {
+            const int g1 = tid / TBQ + turn * (NT / TBQ);
+            const int coil1 = g1 / R2, n2 = g1 - coil1 * R2;
+            if (coil1 >= 4) break;
+            const int slot1 = Q::slot(coil1, col1, n2);
             float2 v[R1];
             if (un.x + coil1 >= a.nch) {
                 // a padding coil of the last quad: zeros
@@ -203,7 +216,11 @@ k_fwd_x_quad(FwdXQuadArgs a, const __grid_constant__ CUtensorMap tmap, int nunit
             fence_proxy_async_smem();
             issue(k + 1);
         }
-        if (act2) {
+#pragma unroll 1
+        for (int turn = 0; turn < Q::T2; ++turn) {
+            const int k1 = tid / W + turn * Q::NG;
+            if (k1 >= R1) break;
+            if (turn > 0) load_mask(mw, un.w, k1);
             float2 u[R2];
 #pragma unroll
             for (int m = 0; m < R2; ++m) u[m] = s_y[(k1 * R2 + m) * W + Q::slot(coil2, col2, m)];
