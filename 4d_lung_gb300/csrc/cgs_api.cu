@@ -149,6 +149,7 @@ struct cgs_ctx {
                                              // over the x passes' (quad grid); -1 not built
     // transposed tap matrix of the listed tiles' points (spreading variant 6)
     bool csr_valid = false;
+    bool no_slices = false;                  // the slices of these bins did not fit (build_slices)
     DevBuf d_col_mark;                       // per bin and grid column: some sample's support reaches it
     bool tile_lists_built = false;           // ensure_tile_lists
     long long csr_pts = 0;
@@ -445,11 +446,62 @@ int upload(cgs_ctx* c, DevBuf& b, const void* h, size_t bytes)
     return CGS_OK;
 }
 
+int csr_list_wanted(const cgs_ctx* c);
+
+// The slices of the ordered rows a.ent (ne taps).  fits: false, with nothing to
+// undo but the buffers, when the device has no room for them beside the rows, or
+// when padding would more than double the rows' memory (a few points with most of
+// a tile's taps; 2^16 entries more are let pass, since few taps mean loose slices).
+// Rows and slices together are the peak of a set-up: 8 bytes a tap, and again
+// 1.1 times that for uniform samples, 1.6 times for 4000 radial spokes.
+int build_slices(cgs_ctx* c, const CsrBuildArgs& a, long long ntl, unsigned long long ne, size_t tmp, bool* fits)
+{
+    *fits = false;
+    SliceArgs sl{};
+    fft_quad_cols(c->G[0], c->lo[0], c->I[0], &sl.R1, &sl.R2);
+    sl.ptr = a.ptr;
+    sl.ent = a.ent;
+    sl.ntl = ntl;
+    sl.tb = a.tb;
+    sl.pts = c->G[0] * a.tb;
+    sl.head_words = slice_head_words(sl.pts);
+    const long long nsl = ntl * (sl.pts / 32), npts = ntl * sl.pts;
+    cudaError_t e = cudaSuccess;
+    auto grow = [&](DevBuf& b, size_t n) {
+        if (e == cudaSuccess) e = b.ensure(n);
+    };
+    grow(c->d_sl_off, (size_t)(nsl + 1) * sizeof(unsigned));
+    grow(c->d_sl_ord, (size_t)npts * sizeof(unsigned short));
+    grow(c->d_sl_head, (size_t)ntl * sl.head_words * sizeof(unsigned));
+    grow(c->d_sl_mask, (size_t)ntl * sl.R2 * a.tb * sizeof(unsigned));
+    if (e == cudaSuccess) {
+        sl.ord = c->d_sl_ord.as<unsigned short>();
+        sl.len = c->d_csr_cnt.as<unsigned>();   // the fill cursors are not needed any more
+        sl.off = c->d_sl_off.as<unsigned>();
+        sl.head = c->d_sl_head.as<unsigned>();
+        sl.lmask = c->d_sl_mask.as<unsigned>();
+        unsigned runs = 0;
+        CGS_CUDA(c, slices_order(sl, c->d_sl_off.as<unsigned>(), c->d_csr_tmp.as<unsigned>(), tmp, &runs, c->stream));
+        if (32ull * runs > 2 * ne + (1u << 16)) return CGS_OK;
+        grow(c->d_sl_ent, std::max<size_t>(runs, 1) * 32 * sizeof(int2));
+    }
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();   // dealt with: later launches do not report it
+        return CGS_OK;
+    }
+    CGS_CUDA(c, e);
+    sl.sell = c->d_sl_ent.as<int2>();
+    CGS_CUDA(c, slices_fill(sl, c->stream));
+    *fits = true;
+    return CGS_OK;
+}
+
 // The transposed tap matrix over the points of the listed tiles of the
 // spreading gather (list 0, variants 6 and 7) or of the x passes (list 1,
 // the gather fused with the adjoint x pass; list 2, in slices), from the current tap records
 // and support lists.  Skipped (the gather variants then fall back to the
-// tiled kernel) when the counts could overflow 32-bit offsets.
+// tiled kernel) when the counts could overflow 32-bit offsets.  Slices that do not
+// fit give way to rows until the bins are next rebuilt.
 int build_csr(cgs_ctx* c, int list)
 {
     c->csr_valid = false;
@@ -494,29 +546,13 @@ int build_csr(cgs_ctx* c, int list)
     a.ent = c->d_csr_ent.as<int2>();
     CGS_CUDA(c, csr_fill_and_order(a, npts, c->stream));
     if (list == 2) {
-        SliceArgs sl{};
-        fft_quad_cols(c->G[0], c->lo[0], c->I[0], &sl.R1, &sl.R2);
-        sl.ptr = a.ptr;
-        sl.ent = a.ent;
-        sl.ntl = ntl;
-        sl.tb = tbx;
-        sl.pts = c->G[0] * tbx;
-        sl.head_words = slice_head_words(sl.pts);
-        const long long nsl = ntl * (sl.pts / 32);
-        CGS_CUDA(c, c->d_sl_off.ensure((size_t)(nsl + 1) * sizeof(unsigned)));
-        CGS_CUDA(c, c->d_sl_ord.ensure((size_t)npts * sizeof(unsigned short)));
-        CGS_CUDA(c, c->d_sl_head.ensure((size_t)ntl * sl.head_words * sizeof(unsigned)));
-        CGS_CUDA(c, c->d_sl_mask.ensure((size_t)ntl * sl.R2 * tbx * sizeof(unsigned)));
-        sl.ord = c->d_sl_ord.as<unsigned short>();
-        sl.len = c->d_csr_cnt.as<unsigned>();   // the fill cursors are not needed any more
-        sl.off = c->d_sl_off.as<unsigned>();
-        sl.head = c->d_sl_head.as<unsigned>();
-        sl.lmask = c->d_sl_mask.as<unsigned>();
-        unsigned runs = 0;
-        CGS_CUDA(c, slices_order(sl, c->d_sl_off.as<unsigned>(), c->d_csr_tmp.as<unsigned>(), tmp, &runs, c->stream));
-        CGS_CUDA(c, c->d_sl_ent.ensure(std::max<size_t>(runs, 1) * 32 * sizeof(int2)));
-        sl.sell = c->d_sl_ent.as<int2>();
-        CGS_CUDA(c, slices_fill(sl, c->stream));
+        bool fits = false;
+        CGS_TRY(build_slices(c, a, ntl, ne, tmp, &fits));
+        if (!fits) {
+            c->no_slices = true;
+            for (DevBuf* b : {&c->d_sl_off, &c->d_sl_ord, &c->d_sl_head, &c->d_sl_mask, &c->d_sl_ent}) b->release();
+            return build_csr(c, csr_list_wanted(c));
+        }
     }
     int bad = 0;
     CGS_CUDA(c, cudaMemcpyAsync(&bad, c->d_flag.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -548,8 +584,12 @@ bool fused_spread_applies(const cgs_ctx* c)
 bool quad_grid(const cgs_ctx* c) { return c->nch >= 3; }
 // The spreading into the quad grid: where at most a third of it is padding
 // (not with five coils, whose second quad holds one: gather and x pass of a
-// 128 x 176 x 96 grid 0.22 ms against 0.20 by rows into coil planes)
-bool quad_spread(const cgs_ctx* c) { return quad_grid(c) && 12 * ((c->nch + 3) / 4) <= 4 * c->nch; }
+// 128 x 176 x 96 grid 0.22 ms against 0.20 by rows into coil planes), unless the
+// slices did not fit
+bool quad_spread(const cgs_ctx* c)
+{
+    return quad_grid(c) && !c->no_slices && 12 * ((c->nch + 3) / 4) <= 4 * c->nch;
+}
 int spread_variant(const cgs_ctx* c) { return c->spread_wpp ? c->spread_wpp : quad_spread(c) ? 6 : 8; }
 // values of a bin's forward grid
 long long fwd_grid_elems(const cgs_ctx* c)
@@ -582,14 +622,20 @@ int build_touch_mask(cgs_ctx* c)
     return CGS_OK;
 }
 
+// form of the matrix that the current spreading variant reads
+int csr_list_wanted(const cgs_ctx* c)
+{
+    const int v = spread_variant(c);
+    return v == 8 && fused_spread_applies(c) ? 1 : v != 7 && quad_spread(c) ? 2 : 0;
+}
+
 // The transposed tap matrix over the listing the current spreading variant
 // reads (rebuilt, and the captured graphs dropped, when it changes)
 int ensure_csr(cgs_ctx* c)
 {
     if (!c->sup_built) return CGS_OK;
-    const int v = spread_variant(c);
-    if (v < 6 && c->csr_valid) return CGS_OK;   // not read by these
-    const int want = v == 8 && fused_spread_applies(c) ? 1 : v != 7 && quad_spread(c) ? 2 : 0;
+    if (spread_variant(c) < 6 && c->csr_valid) return CGS_OK;   // not read by these
+    const int want = csr_list_wanted(c);
     if (c->csr_list == want && c->csr_valid) return CGS_OK;
     drop_graphs(c);
     return build_csr(c, want);
@@ -712,6 +758,7 @@ int rebuild_bins(cgs_ctx* c)
     t0 = clk::now();
     c->csr_list = -1;
     c->csr_valid = false;
+    c->no_slices = false;
     c->touch_words = 0;
     CGS_TRY(ensure_csr(c));
     CGS_TRY(build_touch_mask(c));
