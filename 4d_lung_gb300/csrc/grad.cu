@@ -247,11 +247,12 @@ CGS_D void quad_taps(const TapRecord* rec, const TapRecord* drec, long long i, i
 }
 
 // (factor, derivative): read where it is used (volatile), so that the compiler
-// does not keep the factors or the taps' weights across the coils
+// does not keep the factors or the taps' weights across the coils; "memory", as
+// the asm reads what quad_taps stored
 CGS_D float2 xy_pair(const QuadTaps& t, int q)
 {
     float2 v;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_addr(t.xy + 2 * q)));
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_addr(t.xy + 2 * q)) : "memory");
     return v;
 }
 
