@@ -281,9 +281,14 @@ struct SizeImpl {
             const long long nstrips = (long long)a.ntb * (batch / nsub);
             if (nstrips <= 0) return cudaSuccess;
             const long long nblk = (long long)sm_count() * (per_sm > 0 ? per_sm : 1);
-            // sub-items of a strip that one unit takes: all of them when that leaves every
-            // block 8 units (a last wave of an eighth at most), fewer on smaller grids
-            const long long want = std::min<long long>(nsub, (8 * nblk + nstrips - 1) / nstrips);
+            // units a strip's sub-items are split into: as many as give every block 2 units,
+            // and 8 (a last wave of an eighth) while a unit keeps 8 sub-items or more over
+            // which its strip of P is read once.  8 units a block at any size made units of
+            // one to three: lines of 256, 3 coils of 2 bins 64 -> 57 us (P staged per tile 55),
+            // 8 coils of lines of 224 133 -> 117 (129); 2 at any size: 20 coils of 4 bins, lines
+            // of 192, 431 -> 440 us
+            const long long want = std::max(std::min<long long>(nsub, (2 * nblk + nstrips - 1) / nstrips),
+                                            std::min<long long>(std::max(nsub / 8, 1), (8 * nblk + nstrips - 1) / nstrips));
             const int gsub = (int)((nsub + want - 1) / want);
             const long long nunits = nstrips * ((nsub + gsub - 1) / gsub);
             k_toep_x_tma<R1, R2, TBT, NST><<<(unsigned)std::min(nblk, nunits), Lay::NT, smem, s>>>(a, P, nsub, gsub, map,
