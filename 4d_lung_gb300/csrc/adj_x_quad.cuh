@@ -55,7 +55,9 @@ k_adj_x_quad(AdjXQuadArgs a, int nunits, int per_quad, int nsub)
     __syncthreads();
     const int nq = (a.nch + 3) / 4;
     // stage 1: coil fastest, then column, then n2; stage 2: column fastest, then k1, then coil
-    const int coil1 = tid & 3, col1 = (tid >> 2) % TBQ, col2 = tid % TBQ;
+    const int coil1 = tid & 3, col1 = (tid >> 2) % TBQ, n2 = tid / W;
+    const int col2 = tid % TBQ, g2 = tid / TBQ;
+    const int coil2a = g2 / R1, k1sa = g2 - coil2a * R1;   // of the first turn
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const int q = u / per_quad, rem = u - q * per_quad;   // quads outer, as the forward pass
         const int t = rem / nsub, s = rem - t * nsub;
@@ -91,7 +93,6 @@ k_adj_x_quad(AdjXQuadArgs a, int nunits, int per_quad, int nsub)
 #pragma unroll
             for (int k1 = 0; k1 < R1; ++k1) s_y[(k1 * R2 + n2) * W + Q::slot(coil1, col1, k1)] = v[k1];
         };
-        const int n2 = tid / W;
         float2 v[R1];
         if (n2 < R2) rows(v, n2);
         // the exchange is free once every thread has left stage 2 of the last unit
@@ -107,8 +108,8 @@ k_adj_x_quad(AdjXQuadArgs a, int nunits, int per_quad, int nsub)
         __syncthreads();
 #pragma unroll 1
         for (int turn = 0; turn < Q::T2; ++turn) {
-            const int g2 = tid / TBQ + turn * (NT / TBQ);
-            const int coil2 = g2 / R1, k1s = g2 - coil2 * R1;
+            const int coil2 = turn == 0 ? coil2a : (g2 + turn * (NT / TBQ)) / R1;
+            const int k1s = turn == 0 ? k1sa : g2 + turn * (NT / TBQ) - coil2 * R1;
             if (coil2 >= nc) break;
             float2 w[R2];
 #pragma unroll

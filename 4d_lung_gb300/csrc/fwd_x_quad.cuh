@@ -129,7 +129,10 @@ k_fwd_x_quad(FwdXQuadArgs a, const __grid_constant__ CUtensorMap tmap, int nunit
     };
 
     // stage 1: column fastest, then n2, then coil; stage 2: coil fastest, then column, then k1
-    const int col1 = tid % TBQ, coil2 = tid & 3, col2 = (tid >> 2) % TBQ;
+    const int col1 = tid % TBQ, g1 = tid / TBQ;
+    const int coil1a = g1 / R2, n2a = g1 - coil1a * R2;   // of the first turn
+    const int slot1a = Q::slot(coil1a & 3, col1, n2a);
+    const int coil2 = tid & 3, col2 = (tid >> 2) % TBQ, k1a = tid / W;
     auto load_mask = [&](uint32_t (&mw)[Q::R2W], int entry, int k1) {
         if (a.mask) {
             const uint32_t* m = a.mask + ((long long)entry * R1 + k1) * Q::R2W;
@@ -166,13 +169,13 @@ k_fwd_x_quad(FwdXQuadArgs a, const __grid_constant__ CUtensorMap tmap, int nunit
         const int4 un = s_unit[k & 1];
         // touch-mask bytes of a row group k1 (one per k2, a bit per column), of the first turn ahead
         uint32_t mw[Q::R2W];
-        load_mask(mw, un.w, tid / W < R1 ? tid / W : 0);
+        load_mask(mw, un.w, k1a < R1 ? k1a : 0);
 #pragma unroll 1
         for (int turn = 0; turn < Q::T1; ++turn) {
-            const int g1 = tid / TBQ + turn * (NT / TBQ);
-            const int coil1 = g1 / R2, n2 = g1 - coil1 * R2;
+            const int coil1 = turn == 0 ? coil1a : (g1 + turn * (NT / TBQ)) / R2;
+            const int n2 = turn == 0 ? n2a : g1 + turn * (NT / TBQ) - coil1 * R2;
             if (coil1 >= 4) break;
-            const int slot1 = Q::slot(coil1, col1, n2);
+            const int slot1 = turn == 0 ? slot1a : Q::slot(coil1, col1, n2);
             float2 v[R1];
             if (un.x + coil1 >= a.nch) {
                 // a padding coil of the last quad: zeros
@@ -218,7 +221,7 @@ k_fwd_x_quad(FwdXQuadArgs a, const __grid_constant__ CUtensorMap tmap, int nunit
         }
 #pragma unroll 1
         for (int turn = 0; turn < Q::T2; ++turn) {
-            const int k1 = tid / W + turn * Q::NG;
+            const int k1 = k1a + turn * Q::NG;
             if (k1 >= R1) break;
             if (turn > 0) load_mask(mw, un.w, k1);
             float2 u[R2];
