@@ -582,10 +582,10 @@ bool fused_spread_applies(const cgs_ctx* c)
 // The forward grid holds quads of coils (fwd_x_quad.cuh) from three coils on;
 // with one or two, coil planes (a quad would be mostly padding).
 bool quad_grid(const cgs_ctx* c) { return c->nch >= 3; }
-// The spreading into the quad grid: where at most a third of it is padding
-// (not with five coils, whose second quad holds one: gather and x pass of a
-// 128 x 176 x 96 grid 0.22 ms against 0.20 by rows into coil planes), unless the
-// slices did not fit
+// The spreading into the quad grid: where the padding is at most a third of the
+// coils, from three on all counts but five, whose second quad holds one (gather
+// and x pass of a 128 x 176 x 96 grid, the one measured: 0.22 ms against 0.20 by
+// rows into coil planes), unless the slices did not fit
 bool quad_spread(const cgs_ctx* c)
 {
     return quad_grid(c) && !c->no_slices && 12 * ((c->nch + 3) / 4) <= 4 * c->nch;

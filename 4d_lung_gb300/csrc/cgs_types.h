@@ -260,7 +260,7 @@ struct CsrSpreadArgs {
 };
 
 // The transposed tap matrix of the listed x-pass tiles in slices: a tile's
-// points in falling order of their tap counts, 32 a slice; tap j of the
+// points in falling order of classes of tap counts, 32 a slice; tap j of the
 // slice's point l at sell[(off + j) * 32 + l], padded with zero weights to the
 // longest of the 32.
 struct SliceArgs {

@@ -738,7 +738,7 @@ __global__ void __launch_bounds__(32 * SQ_WARPS, KAHAN ? 4 : 6) k_spread_quad(Sl
     for (int sl = warp; sl < a.pts / 32; sl += SQ_WARPS) {
         const unsigned o0 = __ldg(head + sl);
         const int n = (int)(__ldg(head + sl + 1) - o0);
-        if (n == 0) break;   // slices come in falling order of length
+        if (n == 0) break;   // the points without taps come last
         const int2* ep = a.sell + (long long)o0 * 32 + lane;
         const int pt = a.ord[J * a.pts + sl * 32 + lane];
         float acc[8], cmp[8];
