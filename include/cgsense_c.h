@@ -322,7 +322,9 @@ int cgs_set_deterministic(cgs_ctx* ctx, int32_t on);
  * block per listed 8-column tile and chunk of spread_cc coils (2, 4 or 6, 0 by
  * the coil count), the grid kept in shared memory -- where the grid is not
  * twice the image along x, or the coil count has no such chunk, variant 6
- * runs.  The default is 6 in its sliced form where that applies, else 8),
+ * runs.  The default is 6 in its sliced form where that applies, else 8; slices
+ * that do not fit the device's memory, or would more than double the rows', give
+ * way to rows until the bins are rebuilt),
  * coils per interpolation thread (1, 2, 4, 6, 8; with coils in quads 6 and
  * 8 count as 4).  Variants 1, 2, 4, 5, 6,
  * 7, 8 and every interpolation shape give bitwise-identical results. */
