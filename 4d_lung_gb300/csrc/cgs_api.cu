@@ -1310,6 +1310,8 @@ int build_toeplitz_psf(cgs_ctx* c, const int nf[3])
         cz.out_off = nf[2] / 2 - I[2];
         cz.tw = tw[2].as<float2>();
         CGS_LAUNCH(c, launch_contig(nf[2], +1, cz, 1, c->stream));
+        CGS_CUDA(c, fft_init(nf[1]));
+        CGS_CUDA(c, fft_init(nf[0]));
         StridedPassArgs sy{};
         sy.in = bufA.as<float2>();
         sy.out = bufB.as<float2>();
@@ -1729,7 +1731,9 @@ int cgs_create(const cgs_params* p, cgs_ctx** out)
     if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess)
         return bad(CGS_ERR_CUDA, "cudaStreamCreate failed");
     c->stream = c->own_stream;
-    if (kernels_init() != cudaSuccess) return bad(CGS_ERR_CUDA, "kernel attribute setup failed");
+    cudaError_t ke = kernels_init();
+    for (int a = 0; a < 3 && ke == cudaSuccess; ++a) ke = fft_init(c->G[a]);
+    if (ke != cudaSuccess) return bad(CGS_ERR_CUDA, "kernel attribute setup failed");
     // tap threshold: convFunction(0) * kb_thresh (Reco.cpp:716-717)
     double kb0 = 1.0;
     for (int a = 0; a < 3; ++a) kb0 *= kb_factor(*p, c->G[a], 0.0);

@@ -24,13 +24,14 @@ static const int kSizes[] = {
     CGS_FFT_SIZES(CGS_LIST)
 };
 
-cudaError_t fft_init_all()
+cudaError_t fft_init(int L)
 {
-    cudaError_t e = cudaSuccess;
-#define CGS_INIT(L_, R1_, R2_, G_) if (e == cudaSuccess) e = fft_init_##L_();
-    CGS_FFT_SIZES(CGS_INIT)
-#undef CGS_INIT
-    return e;
+    switch (L) {
+#define CGS_CASE(L_, R1_, R2_, G_) case L_: return fft_init_##L_();
+        CGS_FFT_SIZES(CGS_CASE)
+#undef CGS_CASE
+    }
+    return cudaErrorInvalidValue;
 }
 
 // cuTensorMapEncodeTiled from the driver (no link-time dependency on libcuda)

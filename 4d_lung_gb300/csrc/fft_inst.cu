@@ -66,11 +66,19 @@ struct SizeImpl {
     static constexpr int TBQ_IN = fft_quad_tile_cols(R1, R2, true), TBQ_NO = fft_quad_tile_cols(R1, R2, false);
     static constexpr int TBQ_ADJ = fft_adj_quad_tile_cols(R1, R2);   // of the adjoint x pass from it
 
+    // dynamic shared memory of a kernel: up to 48 KiB with its static part it needs
+    // no attribute
+    template <class F>
+    static cudaError_t dyn_smem(F* f, size_t bytes)
+    {
+        if (bytes <= 46 * 1024) return cudaSuccess;
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    }
+
     template <int SIGN, int MODE, int TBK = TB, int NS = NSTAGE>
     static cudaError_t tma_attr(int smem)
     {
-        return cudaFuncSetAttribute(k_fft_strided_tma<R1, R2, SIGN, TBK, NS, MODE>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        return dyn_smem(k_fft_strided_tma<R1, R2, SIGN, TBK, NS, MODE>, smem);
     }
 
     static cudaError_t init()
@@ -89,27 +97,18 @@ struct SizeImpl {
                 e = tma_attr<+1, PRUNE_OUT, TBN>((int)PipeLayout<R1, R2, TBN, NSTAGE>::smem_bytes(L));
         }
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_fwd_x_quad<R1, R2, TBQ_NO, PRUNE_NONE>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)QuadLayout<R1, R2, TBQ_NO>::smem_bytes(L + 3));
+            e = dyn_smem(k_fwd_x_quad<R1, R2, TBQ_NO, PRUNE_NONE>, QuadLayout<R1, R2, TBQ_NO>::smem_bytes(L + 3));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_adj_x_quad<R1, R2, TBQ_ADJ, PRUNE_NONE>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)AdjQuadLayout<R1, R2, TBQ_ADJ>::smem_bytes);
+            e = dyn_smem(k_adj_x_quad<R1, R2, TBQ_ADJ, PRUNE_NONE>, AdjQuadLayout<R1, R2, TBQ_ADJ>::smem_bytes);
         if constexpr (HAS_OUT)
             if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_adj_x_quad<R1, R2, TBQ_ADJ, PRUNE_OUT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)AdjQuadLayout<R1, R2, TBQ_ADJ>::smem_bytes);
+                e = dyn_smem(k_adj_x_quad<R1, R2, TBQ_ADJ, PRUNE_OUT>, AdjQuadLayout<R1, R2, TBQ_ADJ>::smem_bytes);
         if constexpr (HAS_IN)
             if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_fwd_x_quad<R1, R2, TBQ_IN, PRUNE_IN>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)QuadLayout<R1, R2, TBQ_IN>::smem_bytes(L / 2));
+                e = dyn_smem(k_fwd_x_quad<R1, R2, TBQ_IN, PRUNE_IN>, QuadLayout<R1, R2, TBQ_IN>::smem_bytes(L / 2));
         if constexpr (HAS_IN)
             if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_toep_x_tma<R1, R2, TBT, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)ToepLayout<R1, R2, TBT, NST>::smem_bytes(L / 2));
+                e = dyn_smem(k_toep_x_tma<R1, R2, TBT, NST>, ToepLayout<R1, R2, TBT, NST>::smem_bytes(L / 2));
         // the z extent of an image never exceeds the grid's: size for Iz = L
         if constexpr (HAS_IN && HAS_OUT) {
             if (e == cudaSuccess) e = sax_attr<2, false>();
@@ -128,16 +127,13 @@ struct SizeImpl {
     template <bool HALF>
     static cudaError_t z_attr()
     {
-        cudaError_t e = cudaFuncSetAttribute(k_fwd_z_pipe<R1, R2, LPB, ZNST_F, false, HALF>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)ZF::smem_bytes(HALF ? L / 2 : L, false, HALF));
+        cudaError_t e = dyn_smem(k_fwd_z_pipe<R1, R2, LPB, ZNST_F, false, HALF>,
+                                 ZF::smem_bytes(HALF ? L / 2 : L, false, HALF));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_fwd_z_pipe<R1, R2, LPB, ZNST_F, true, HALF>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)ZF::smem_bytes(HALF ? L / 2 : L, false, HALF));
+            e = dyn_smem(k_fwd_z_pipe<R1, R2, LPB, ZNST_F, true, HALF>,
+                         ZF::smem_bytes(HALF ? L / 2 : L, false, HALF));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_adj_z_pipe<R1, R2, LPB, ZNST_A, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)ZA::smem_bytes(HALF ? L / 2 : L, true, HALF));
+            e = dyn_smem(k_adj_z_pipe<R1, R2, LPB, ZNST_A, HALF>, ZA::smem_bytes(HALF ? L / 2 : L, true, HALF));
         return e;
     }
 

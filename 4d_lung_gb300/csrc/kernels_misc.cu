@@ -224,7 +224,6 @@ cudaError_t kernels_init()
                             (const void*)k_spread_pipe<4, 2>, (const void*)k_spread_pipe<6, 2>};
     for (int i = 0; i < 6 && e == cudaSuccess; ++i)
         e = cudaFuncSetAttribute(pipes[i], cudaFuncAttributeMaxDynamicSharedMemorySize, spp);
-    if (e == cudaSuccess) e = fft_init_all();
     return e;
 }
 

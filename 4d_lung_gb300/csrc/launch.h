@@ -11,8 +11,11 @@ namespace cgs {
 // Supported line lengths of the 3-D FFT (each a product R1*R2 of two
 // register codelets).  Grid sizes must be taken from this list.
 bool fft_supported(int L);
-// per-device kernel attributes of the FFT passes (dynamic shared memory)
-cudaError_t fft_init_all();
+// kernel attributes (dynamic shared memory) of the FFT passes of one line length on
+// the current device, to be set before their first launch.  A context sets those
+// of its own lengths: all 20 cost each new context 100 us more and the first one
+// of a process 17 ms, in which their kernels were loaded
+cudaError_t fft_init(int L);
 // 4-D tensor map [batch][A][Lin][B] of a strided pass's input with a
 // TB x box_rows box; false when the buffer or strides are not 16-byte aligned.
 // promo: L2 promotion of the box's rows in bytes (64, 128 or 256)
